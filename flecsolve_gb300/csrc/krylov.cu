@@ -1205,6 +1205,10 @@ static int k_default(const Solver *s) {
 
 static int cg_apply64(Solver *s, Vec *b, Vec *x, fs_solve_info *info) {
 	Ctx *ctx = s->ctx;
+	int taken = 0;
+	FS_TRY(cg_apply_resident(s, b, x, info, &taken));
+	if (taken)
+		return FS_OK;
 	const int64_t n = s->n;
 	const int G = red_grid(ctx, n);
 	const bool zg = s->set.base.use_zero_guess != 0;

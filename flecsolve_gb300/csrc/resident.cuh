@@ -1,0 +1,477 @@
+// Grid-resident solver kernels: a whole solve (or its iteration loop) in one
+// cooperative launch.
+//
+// A Krylov iteration of a system whose vectors fit in the shared memories and
+// the L2 is a chain of short phases separated by reductions.  As separate
+// kernels each phase costs its launch, the ramp of its CTAs and a last-CTA
+// fold: 20.8 us an iteration for FP64 CG on 16,384 rows, of which the
+// arithmetic is under 1 us.  Here one CTA per SM owns a contiguous slice of
+// the rows for the whole solve, and the CTAs meet through messages alone:
+//
+//  * grid_sum, a reduction: every CTA stores one 16-byte message per value,
+//    {sum, epoch}, in a slot of its own and reads all slots until they carry
+//    the epoch -- one store and one load through the L2, the value and its
+//    flag in one access.  Every CTA forms the same sum.  Two slot sets
+//    alternate: a CTA overwrites a slot two epochs later, after every CTA has
+//    sent the message between, that is, has read the older one.
+//  * packets, a vector's neighbour rows: each row of the vector is stored as
+//    {value, epoch}, and a slice that needs a row of another one reads it
+//    until it carries the epoch.  No fence and no barrier stand between the
+//    writer and the reader.
+//
+// The launch is cooperative, so all CTAs are resident and every wait ends; as
+// a guard the waits are bounded all the same (kResPolls reads, a second or
+// more), after which the CTA records an error in the context's device error
+// word and leaves, as do the others when their own waits run out.
+#pragma once
+
+#include "solver.cuh"
+
+namespace fsg {
+
+constexpr int kResMaxG = 160;      // CTAs of a resident grid at most
+constexpr int kResMaxVals = 4;     // values per grid_sum at most
+constexpr int kResThreads = 512;   // threads per CTA at most
+constexpr int kResPolls = 1 << 22;
+
+// ------------------------------------------------ sums in fixed point --
+//
+// A warp's FP64 instruction occupies its scheduler for 63 cycles on this GPU
+// whether or not it depends on the last (measured; 19 cycles an instruction
+// an SM with 16 warps), so a tree of shuffles and adds over the warp, the CTA
+// and the grid costs more than the messages do: 2,193 cycles of a one-CTA
+// sum, of which the message was 600.  The sums therefore run in integers: every
+// value is aligned to the largest exponent of its group, its magnitude cut
+// into four 23-bit pieces of a 96-bit window, and the pieces are added with
+// redux.sync (at most 256 values: 23 + 8 bits).  A value loses only bits
+// below 2^-30 of the unit in the last place of the group's largest value, a
+// warp's sum is rounded to an eighth of that unit and a CTA's to the unit, so
+// the result is at least as accurate as the tree's, and it does not depend on
+// the order of the values.
+
+// a group's sum q 2^(e - 1075 - F), F = 3 for a warp, 0 for a CTA; e = 0x7ff:
+// some value was not finite, q the union of 1 (+inf), 2 (-inf) and 4 (NaN)
+struct ResFix {
+	long long q;
+	int e;
+};
+
+struct ResPieces {
+	int p[4];
+	__device__ __forceinline__ void clear() {
+#pragma unroll
+		for (int i = 0; i < 4; ++i)
+			p[i] = 0;
+	}
+	// adds m (m < 2^62; -m when neg) shifted right by d >= 0: the window is
+	// m 2^34 / 2^d, its bits 73.., 50.., 27.. and 4.. the pieces
+	__device__ __forceinline__ void add(unsigned long long m, int d, bool neg) {
+		m <<= 2;
+		unsigned w2 = (unsigned)(m >> 32), w1 = (unsigned)m, w0 = 0;
+		if (d >= 32) {
+			w0 = d < 64 ? w1 : d < 96 ? w2 : 0u;
+			w1 = d < 64 ? w2 : 0u;
+			w2 = 0;
+		}
+		const int r = d & 31;
+		w0 = __funnelshift_r(w0, w1, r);
+		w1 = __funnelshift_r(w1, w2, r);
+		w2 >>= r;
+		constexpr unsigned M = (1u << 23) - 1;
+		const int v[4] = {(int)(w2 >> 9), (int)(__funnelshift_r(w1, w2, 18) & M),
+		                  (int)(__funnelshift_r(w0, w1, 27) & M), (int)((w0 >> 4) & M)};
+#pragma unroll
+		for (int i = 0; i < 4; ++i)
+			p[i] += neg ? -v[i] : v[i];
+	}
+	__device__ __forceinline__ void warp_sum() {
+#pragma unroll
+		for (int i = 0; i < 4; ++i)
+			p[i] = __reduce_add_sync(0xffffffffu, p[i]);
+	}
+	// the sum as hi 2^16 + lo 2^-30 in the units of m, 0 <= lo < 2^46
+	__device__ __forceinline__ void split(long long &hi, long long &lo) const {
+		hi = (long long)p[0] * (1 << 23) + p[1];
+		lo = (long long)p[2] * (1 << 23) + p[3];
+		hi += lo >> 46;
+		lo &= (1ll << 46) - 1;
+	}
+};
+
+__device__ __forceinline__ ResFix res_special(int cls) {
+	return {(long long)__reduce_or_sync(0xffffffffu, (unsigned)cls), 0x7ff};
+}
+
+// the sum of a warp's 32 doubles, F = 3
+__device__ __forceinline__ ResFix res_fix_warp(double v) {
+	const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+	int e = (int)(bits >> 52) & 0x7ff;
+	unsigned long long m = bits & ((1ull << 52) - 1);
+	const bool neg = bits >> 63;
+	const int E = __reduce_max_sync(0xffffffffu, max(e, 1));
+	if (E == 0x7ff)
+		return res_special(e != 0x7ff ? 0 : m ? 4 : neg ? 2 : 1);
+	if (e)
+		m |= 1ull << 52;
+	else
+		e = 1;
+	ResPieces s;
+	s.clear();
+	s.add(m, E - e, neg);
+	s.warp_sum();
+	long long hi, lo;
+	s.split(hi, lo);
+	return {hi * (1 << 19) + ((lo + (1ll << 26)) >> 27), E};
+}
+
+// the sum of the warps' sums (one a lane, {0, 1} in idle lanes), F = 0
+__device__ __forceinline__ ResFix res_fix_cta(ResFix f) {
+	const int E = __reduce_max_sync(0xffffffffu, f.e);
+	if (E == 0x7ff)
+		return res_special(f.e == 0x7ff ? (int)f.q : 0);
+	ResPieces s;
+	s.clear();
+	s.add((unsigned long long)(f.q < 0 ? -f.q : f.q), E - f.e, f.q < 0);
+	s.warp_sum();
+	long long hi, lo;
+	s.split(hi, lo);
+	return {hi * (1 << 13) + ((lo + (1ll << 32)) >> 33), E};
+}
+
+// the sum of the CTAs' sums, Q a lane, as a double (the same in every lane)
+template<int Q>
+__device__ __forceinline__ double res_fix_grid(const ResFix (&f)[Q]) {
+	int E = 1;
+#pragma unroll
+	for (int i = 0; i < Q; ++i)
+		E = max(E, f[i].e);
+	E = __reduce_max_sync(0xffffffffu, E);
+	if (E == 0x7ff) {
+		int cls = 0;
+#pragma unroll
+		for (int i = 0; i < Q; ++i)
+			cls |= f[i].e == 0x7ff ? (int)f[i].q : 0;
+		const long long q = res_special(cls).q;
+		const double inf = __longlong_as_double(0x7ff0000000000000ll);
+		return (q & 4) || (q & 3) == 3 ? __longlong_as_double(0x7ff8000000000000ll)
+		                               : (q & 1) ? inf : -inf;
+	}
+	ResPieces s;
+	s.clear();
+#pragma unroll
+	for (int i = 0; i < Q; ++i)
+		s.add((unsigned long long)(f[i].q < 0 ? -f[i].q : f[i].q), E - f[i].e, f[i].q < 0);
+	s.warp_sum();
+	long long hi, lo;
+	s.split(hi, lo);
+	// (hi + lo 2^-46) 2^(E - 1059)
+	const double t = fma((double)lo, 0x1p-46, (double)hi);
+	const int k = E - 1059;
+	if (k >= -1022)
+		return t * __longlong_as_double((long long)(k + 1023) << 52);
+	return t * 0x1p-600 * __longlong_as_double((long long)(k + 600 + 1023) << 52);
+}
+
+// ------------------------------------------------------------ messages --
+
+// device memory of the messages: two sets of kResMaxVals x kResMaxG slots
+// {sum, epoch << 16 | exponent}, then the epoch reached by the last launch
+struct ResSlots {
+	ulonglong2 msg[2][kResMaxVals][kResMaxG];
+	unsigned long long epoch;
+};
+
+struct ResShared {
+	ResFix part[kResMaxVals][kResThreads / 32];
+	double bc[8];  // scalars handed from warp 0 to the CTA
+	int stop;      // set by warp 0: leave the iteration loop
+	int fail;      // a wait ran out
+};
+
+__device__ __forceinline__ void res_st16(ulonglong2 *p, unsigned long long a, unsigned long long b) {
+	asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(p),
+	             "l"(a), "l"(b)
+	             : "memory");
+}
+// the same store as an exchange at the L2: a plain store to a line that other
+// SMs are already polling costs them 2,000 to 4,000 cycles (152 CTAs that
+// arrive 400 to 1,300 cycles apart: 5,760 cycles a round with st, 3,074 with
+// the exchange, 2,419 with the first read held back as well)
+__device__ __forceinline__ void res_xchg16(ulonglong2 *p, unsigned long long a, unsigned long long b) {
+	asm volatile("{\n .reg .b128 t, u;\n mov.b128 t, {%1, %2};\n"
+	             " atom.relaxed.gpu.global.exch.b128 u, [%0], t;\n}\n" ::"l"(p),
+	             "l"(a), "l"(b)
+	             : "memory");
+}
+// cycles from a CTA's own message to its first look at the others': about
+// what a message takes
+constexpr int kResFirstLook = 450;
+__device__ __forceinline__ void res_hold(long long since) {
+	while (clock64() - since < kResFirstLook) {
+	}
+}
+__device__ __forceinline__ ulonglong2 res_ld16(const ulonglong2 *p) {
+	ulonglong2 v;
+	asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}\n"
+	             : "=l"(v.x), "=l"(v.y)
+	             : "l"(p)
+	             : "memory");
+	return v;
+}
+
+// A CTA's view of the resident grid
+struct ResTeam {
+	ResSlots *slots;
+	ResShared *sh;
+	unsigned *err;
+	unsigned long long epoch;  // the same in every thread of the grid
+
+	__device__ void init(ResSlots *s, ResShared *shared, unsigned *e) {
+		slots = s;
+		sh = shared;
+		err = e;
+		epoch = *(volatile unsigned long long *)&s->epoch;
+		if (threadIdx.x == 0) {
+			sh->stop = 0;
+			sh->fail = 0;
+		}
+	}
+	__device__ void failed() {
+		atomicOr(err, 0x40u);
+		*(volatile int *)&sh->fail = 1;
+	}
+
+	// Sums NV values over the grid.  Every thread calls it; warp k carries
+	// value k through the messages (in parallel: two values take a third
+	// longer than one) and has its total in every lane of the returned
+	// value.  Thread 32 k then forms the scalars that follow from it, and
+	// every thread ends the step with done().  PUB: what the CTAs wrote to
+	// global memory before the call is visible to all after done().
+	template<int NV, bool PUB>
+	__device__ double grid_sum(const double (&v)[NV]) {
+		const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+		++epoch;
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			const ResFix f = res_fix_warp(v[k]);
+			if (lane == 0)
+				sh->part[k][wid] = f;
+		}
+		__syncthreads();
+		if (wid >= NV)
+			return 0.0;
+		const int nw = (int)blockDim.x >> 5;
+		ulonglong2 *set = slots->msg[epoch & 1][wid];
+		if (PUB)
+			__threadfence();
+		ResFix own{0, 1};
+		if (lane < nw)
+			own = sh->part[wid][lane];
+		own = res_fix_cta(own);
+		if (lane == 0)
+			res_xchg16(&set[blockIdx.x], (unsigned long long)own.q,
+			           epoch << 16 | (unsigned long long)own.e);
+		res_hold(clock64());
+		constexpr int Q = kResMaxG / 32;
+		const int G = (int)gridDim.x;
+		ResFix f[Q];
+		bool here = false;
+		for (int it = 0; !here && it < kResPolls; ++it) {
+			// every slot of this lane in flight, then the tags
+			ulonglong2 m[Q];
+#pragma unroll
+			for (int q = 0; q < Q; ++q)
+				if (q * 32 < G)
+					m[q] = res_ld16(&set[min(q * 32 + lane, G - 1)]);
+			here = true;
+#pragma unroll
+			for (int q = 0; q < Q; ++q)
+				if (q * 32 < G) {
+					here = here && m[q].y >> 16 == epoch;
+					f[q] = {(long long)m[q].x, (int)(m[q].y & 0xffff)};
+				}
+		}
+#pragma unroll
+		for (int q = 0; q < Q; ++q)
+			if (q * 32 + lane >= G)
+				f[q] = {0, 1};
+		if (!__all_sync(0xffffffffu, here) && lane == 0)
+			failed();
+		const double t = res_fix_grid<Q>(f);
+		if (PUB)
+			__threadfence();
+		return t;
+	}
+	// ends the step; false when a wait ran out (the same in every thread)
+	__device__ bool done() {
+		__syncthreads();
+		return *(volatile int *)&sh->fail == 0;
+	}
+	// the last call of a kernel: the next launch goes on from this epoch
+	// (past every message and packet of this one, also after a failed wait)
+	__device__ void finish() {
+		if (blockIdx.x == 0 && threadIdx.x == 0)
+			slots->epoch = epoch + 16;
+	}
+};
+
+// the largest s with sqrt(s) < tol (below 0 when there is none): the stopping
+// test on a norm without its square root
+__device__ __forceinline__ double res_threshold(double tol) {
+	if (!(tol > 0.0))
+		return -1.0;
+	if (isinf(tol))
+		return 1.7976931348623157e308;
+	double t = fmin(tol * tol, 1.7976931348623157e308);
+	for (int i = 0; i < 8 && t > 0.0 && !(sqrt(t) < tol); ++i)
+		t = __longlong_as_double(__double_as_longlong(t) - 1);
+	for (int i = 0; i < 8; ++i) {
+		const double u = __longlong_as_double(__double_as_longlong(t) + 1);
+		if (!(sqrt(u) < tol))
+			break;
+		t = u;
+	}
+	return t;
+}
+
+// a / b, correctly rounded, from y = 1 / b correctly rounded (Markstein 1990:
+// the residual of a y corrects it); three dependent operations after a is
+// known where a division takes 561 cycles.  Outside the range where the
+// residual is exact it divides.
+__device__ __forceinline__ double res_quotient(double a, double b, double y) {
+	const double q = a * y;
+	const double r = fma(fma(-q, b, a), y, q);
+	const double m = fabs(a), n = fabs(b);
+	const bool safe = m > 0x1p-900 && m < 0x1p900 && n > 0x1p-900 && n < 0x1p900 && fabs(q) > 0x1p-900 &&
+	                  fabs(q) < 0x1p900;
+	return safe ? r : a / b;
+}
+
+// Grid-stencil operator of a resident kernel: the symmetric or the general
+// grid storage (rows addressed by grid coordinates), K = 1..3 dimensions.
+template<class V>
+struct ResGrid {
+	const V *S;
+	int64_t ld;
+	int n, nx, ny, nz;
+};
+
+// per row, the neighbours inside the grid: bits z-, y-, x-, x+, y+, z+
+template<int K>
+__device__ __forceinline__ unsigned res_mask(int r, int nx, int ny, int nz) {
+	const int line = r / nx, i = r - line * nx;
+	const int kk = K >= 3 ? line / ny : 0, j = K >= 2 ? line - kk * ny : 0;
+	unsigned m = 0;
+	if (K >= 3 && kk > 0)
+		m |= 1u;
+	if (K >= 2 && j > 0)
+		m |= 2u;
+	if (i > 0)
+		m |= 4u;
+	if (i < nx - 1)
+		m |= 8u;
+	if (K >= 2 && j < ny - 1)
+		m |= 16u;
+	if (K >= 3 && kk < nz - 1)
+		m |= 32u;
+	return m;
+}
+
+// A slice's operator: the diagonals of the own rows (in shared memory when
+// they fit, else global), the global ones for lower partners outside it
+template<class V, int K, bool GEN>
+struct ResRows {
+	const V *D, *U[3], *L[3];  // own rows, indexed from the slice's first row
+	const V *G;                // symmetric storage: upper diagonals of all rows
+	int64_t ld;
+	int lo, cnt, d[3];         // offsets 1, nx, nx ny
+	const unsigned char *mask;
+
+	// sum of the own row l over a vector whose own rows are vl (indexed from
+	// the slice's first row); rows of other slices come from packets `pk`
+	// carrying `tag` (PKT) or from the global vector vg
+	template<bool PKT>
+	__device__ __forceinline__ V sum(int l, const V *vl, const V *vg, const ulonglong2 *pk,
+	                                 unsigned long long tag, ResTeam &tm) const {
+		const unsigned m = mask[l];
+		V c[2 * K + 1], x[2 * K + 1];
+		ulonglong2 w[2 * K];
+		bool in[2 * K];
+		auto at = [&](int t, int slot, int j) {
+			in[t] = (unsigned)j < (unsigned)cnt;
+			if constexpr (PKT) {
+				if (in[t])
+					x[slot] = vl[j];
+				else
+					w[t] = res_ld16(pk + (lo + j));
+			}
+			else {
+				const V *q = in[t] ? vl + j : vg + (lo + j);
+				x[slot] = *q;
+			}
+		};
+#pragma unroll
+		for (int t = 0; t < K; ++t) {
+			// lower neighbour of offset d[K - 1 - t], upper neighbour of d[t];
+			// an absent one reads the own row and its term is not added
+			const int e = K - 1 - t;
+			const bool lower = m >> (2 - e) & 1, upper = m >> (3 + t) & 1;
+			const int jl = lower ? l - d[e] : l, ju = upper ? l + d[t] : l;
+			at(t, t, jl);
+			at(K + t, K + 1 + t, ju);
+			if (GEN)
+				c[t] = L[e][l];
+			else {
+				const V *q = jl >= 0 ? U[e] + jl : G + ((int64_t)e * ld + lo + jl);
+				c[t] = *q;
+			}
+			c[K + 1 + t] = U[t][l];
+		}
+		x[K] = vl[l];
+		c[K] = D[l];
+		if constexpr (PKT) {
+#pragma unroll
+			for (int t = 0; t < 2 * K; ++t)
+				if (!in[t]) {
+					const int slot = t < K ? t : t + 1;
+					for (int it = 0; w[t].y != tag; ++it) {
+						if (it >= kResPolls || *(volatile int *)&tm.sh->fail) {
+							tm.failed();
+							break;
+						}
+						const int e = t < K ? K - 1 - t : t - K;
+						w[t] = res_ld16(pk + (lo + (t < K ? l - d[e] : l + d[e])));
+					}
+					x[slot] = (V)__longlong_as_double((long long)w[t].x);
+				}
+		}
+		V s = V(0);
+#pragma unroll
+		for (int t = 0; t < K; ++t)
+			s = (m >> (2 - (K - 1 - t)) & 1) ? fma(c[t], x[t], s) : s;
+		s = fma(c[K], x[K], s);
+#pragma unroll
+		for (int t = 0; t < K; ++t)
+			s = (m >> (3 + t) & 1) ? fma(c[K + 1 + t], x[K + 1 + t], s) : s;
+		return s;
+	}
+};
+
+// Hands out the CTA's dynamic shared memory to the slice's arrays in order of
+// use until it is full; an array that does not fit stays where it is.
+struct ResSmem {
+	unsigned char *at;
+	int left;
+	template<class T>
+	__device__ T *take(int count) {
+		const int bytes = (count * (int)sizeof(T) + 15) & ~15;
+		if (bytes > left)
+			return nullptr;
+		T *p = reinterpret_cast<T *>(at);
+		at += bytes;
+		left -= bytes;
+		return p;
+	}
+};
+
+}  // namespace fsg

@@ -68,6 +68,7 @@ struct GmState {
 };
 
 struct Solver;
+struct ResSlots;
 
 struct Precond {
 	int kind = FS_PRECOND_NONE;
@@ -117,6 +118,9 @@ struct Solver {
 	int hist_cap = 0;
 	double *part = nullptr;           // reduction partials
 	unsigned *counter = nullptr;
+	// messages and row packets of the resident kernels (on first use)
+	ResSlots *res_slots = nullptr;
+	ulonglong2 *res_pk = nullptr;
 	// captured graphs, keyed by the operator they were captured with and the
 	// vectors / body they run; at most kMaxGraphs are kept (least recently
 	// launched evicted first)
@@ -154,6 +158,10 @@ int solver_norms(Solver *s, Vec *b, Vec *x, bool with_x, int gmres_rule);
 int solver_hist(Solver *s, int cap);
 int ensure_val32(Csr *A);
 int ensure_dinv(Csr *A);
+
+// a whole solve in one cooperative launch (resident.cu); *taken = 0: not a
+// solve for it, nothing was done
+int cg_apply_resident(Solver *s, Vec *b, Vec *x, fs_solve_info *info, int *taken);
 
 // host-stepped loops for operators and preconditioners the fused device
 // loops do not take (generic.cu)
