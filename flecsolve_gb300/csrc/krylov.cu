@@ -2317,6 +2317,12 @@ FS_API int fs_krylov_apply_transpose(fs_solver h, fs_vec bh, fs_vec xh, fs_solve
 	if (!ok_slv(s))
 		return FS_ERR_BAD_HANDLE;
 	Csr *A = s->A;
+	FS_TRY(reject_matrix_free(A, "transpose"));
+	// a matrix that is symmetric bit for bit is its own transpose: its own
+	// storage serves (no column view built or refreshed)
+	FS_TRY(ensure_sym(A, false));
+	if (A->sym_state == 1)
+		return fs_krylov_apply(h, bh, xh, info);
 	FS_TRY(ensure_transpose(A));
 	FS_TRY(ensure_dinv(A));
 	if (!s->AT) {

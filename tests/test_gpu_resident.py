@@ -114,3 +114,22 @@ def test_resident_cg_reports_non_finite(ctx):
         with pytest.raises(FsError) as e:
             _solve(ctx, A, b, "cg", coding, maxiter=50, rtol=1e-9)
         assert e.value.status == 5
+
+
+@pytest.mark.parametrize("n", [9, 32, 65])
+def test_transpose_solve_of_a_symmetric_matrix_is_the_forward_solve(ctx, n):
+    A = P.diffusion(3, n, seed=3)
+    dA = fs.CSR(ctx, A)
+    vb, vx, vt = fs.Vector(ctx, P.uniform(8, A.nrows)), fs.Vector(ctx, A.nrows), fs.Vector(ctx, A.nrows)
+    slv = fs.cg.solver(fs.cg.settings(maxiter=2000, rtol=1e-10))(fs.op.ref(dA), fs.op.jacobi)
+    a = slv(vb, vx)
+    t = slv.apply_transpose(vb, vt)
+    assert (a.status, a.iters) == (t.status, t.iters)
+    assert np.array_equal(vx.numpy(), vt.numpy())
+    # values that stop being symmetric take the column view again
+    v = A.val.copy()
+    v[1] *= 1.0 + 1e-3
+    dA.update_values(v)
+    slv.apply_transpose(vb, vt)
+    r = vb.numpy() - P.CSR(A.nrows, A.ncols, A.rowptr, A.col, v).to_scipy().T @ vt.numpy()
+    assert np.linalg.norm(r) <= 1e-8 * np.linalg.norm(vb.numpy())
