@@ -17,7 +17,7 @@
 #include <cmath>
 #include <cstring>
 
-#include "solver.cuh"
+#include "resident.cuh"
 
 namespace fsg {
 
@@ -181,32 +181,36 @@ __device__ void finish_step(GmState *g, KState *st, double *hist) {
 	}
 }
 
-// finish_step by the whole CTA: the column H(0..k+1, k) and the k earlier
-// rotations are staged in shared memory (`col`, 3 (k + 2) doubles) by all
-// threads, thread 0 runs the same rotations and tests on them, and the
-// column is written back by all threads -- the serial chain of global
-// loads and stores of the one-thread form costs a few microseconds per
-// rotation at large k.  Every thread of the CTA calls it.
-__device__ void finish_step_cta(GmState *g, KState *st, double *hist, double *col) {
-	const int k = g->k, ld = g->ld, tid = threadIdx.x;
+// finish_step by one warp: the column H(0..k+1, k) and the k earlier
+// rotations are staged in shared memory (`col`, 3 (k + 2) doubles), then lanes
+// 0 and 1 apply the rotations, one row of each rotation a lane (c x + s y and
+// -s x + c y): a product and an FMA a rotation, where one thread issues four
+// FP64 instructions of 62 cycles each.  Every lane of the warp calls it.
+__device__ void finish_step_warp(GmState *g, KState *st, double *hist, double *col) {
+	const int k = g->k, ld = g->ld, lane = threadIdx.x & 31;
 	double *cs = col + (k + 2), *sn = cs + (k + 2);
-	for (int i = tid; i <= k + 1; i += blockDim.x)
+	for (int i = lane; i <= k + 1; i += 32)
 		col[i] = g->H[i + ld * k];
-	for (int i = tid; i < k; i += blockDim.x) {
+	for (int i = lane; i < k; i += 32) {
 		cs[i] = g->cs[i];
 		sn[i] = g->sn[i];
 	}
-	__syncthreads();
-	if (tid == 0) {
-		// the rotations of apply_givens / compute_givens, on the staged column
-		for (int i = 0; i < k; i++) {
-			const double x = col[i], y = col[i + 1], c = cs[i], s = sn[i];
-			col[i] = c * x + s * y;
-			col[i + 1] = -s * x + c * y;
-		}
+	__syncwarp();
+	// x: the upper entry of the rotation, in both lanes
+	double x = col[0];
+	for (int i = 0; i < k; ++i) {
+		const double y = col[i + 1], c = cs[i], s = sn[i];
+		// lane 0: c x + s y; lane 1 (and the others): -s x + c y
+		const double a = lane == 0 ? c : -s, b = lane == 0 ? s : c;
+		const double v = a * x + b * y;
+		if (lane == 0)
+			col[i] = v;
+		x = __shfl_sync(0xffffffffu, v, 1);
+	}
+	if (lane == 0) {
 		const double vnorm = g->vnorm;
 		if (vnorm != 0.0) {
-			const double f = col[k], gg = col[k + 1];
+			const double f = x, gg = col[k + 1];
 			double c, s;
 			if (gg == 0.0) {
 				c = 1.0;
@@ -226,10 +230,12 @@ __device__ void finish_step_cta(GmState *g, KState *st, double *hist, double *co
 			g->sn[k] = s;
 			col[k] = c * f + s * gg;
 			col[k + 1] = 0.0;
-			const double x = g->dw[k];
-			g->dw[k] = c * x;
-			g->dw[k + 1] = -s * x;
+			const double w = g->dw[k];
+			g->dw[k] = c * w;
+			g->dw[k + 1] = -s * w;
 		}
+		else
+			col[k] = x;
 		const double res = fabs(g->dw[k + 1]);
 		g->k = k + 1;
 		const int it = st->iter + 1;
@@ -253,10 +259,10 @@ __device__ void finish_step_cta(GmState *g, KState *st, double *hist, double *co
 			st->flags |= KF_RESTART;
 		}
 	}
-	__syncthreads();
-	for (int i = tid; i <= k + 1; i += blockDim.x)
+	__syncwarp();
+	for (int i = lane; i <= k + 1; i += 32)
 		g->H[i + ld * k] = col[i];
-	__syncthreads();
+	__syncwarp();
 }
 
 // gmres.hh:333-348, nr = k - 1
@@ -810,6 +816,35 @@ int gm_body(Solver *s, void *a) {
 	return FS_OK;
 }
 
+// what the state read back says of the finished solve (gmres.hh:235-242)
+int gmres_info(Solver *s, bool zg, bool mixed, int user_stop, double xn, fs_solve_info *info) {
+	Ctx *ctx = s->ctx;
+	KState &h = *s->hst;
+	s->hhist_count = std::min<int64_t>(h.nhist, s->hist_cap);
+	s->mixed_outer = mixed ? h.restarts : 0;
+	s->mixed_inner = mixed ? h.iter : 0;
+	memset(info, 0, sizeof(*info));
+	info->rhs_norm = (float)h.rhs_norm;
+	info->sol_norm_initial = zg ? 0.f : (float)h.sol0;
+	info->res_norm_initial = (float)h.res0;
+	info->res_norm_final = (float)h.res;
+	info->sol_norm_final = (float)xn;
+	info->restarts = h.restarts;
+	if (user_stop) {
+		info->status = FS_CONVERGED_USER;
+		info->iters = user_stop;
+	}
+	else {
+		info->status = h.status;
+		info->iters = h.info_iters;
+		if (h.res0 >= h.tol && info->iters == 0)
+			info->status = FS_DIVERGED_ITERS;  // gmres.hh:237-238
+	}
+	if (h.flags & KF_NONFINITE)
+		return set_err(ctx, FS_ERR_NON_FINITE, "GMRES: non-finite residual norm");
+	return FS_OK;
+}
+
 template<class T>
 int gmres_run(Solver *s, Vec *b, Vec *x, fs_solve_info *info, bool mixed) {
 	Ctx *ctx = s->ctx;
@@ -938,32 +973,9 @@ int gmres_run(Solver *s, Vec *b, Vec *x, fs_solve_info *info, bool mixed) {
 		FS_TRY(check_launch(ctx, "gmres correct"));
 	}
 	FS_TRY(read_state(s));
-	KState &h = *s->hst;
-	s->hhist_count = std::min<int64_t>(h.nhist, s->hist_cap);
-	s->mixed_outer = mixed ? h.restarts : 0;
-	s->mixed_inner = mixed ? h.iter : 0;
 	double xn = 0;
 	FS_TRY(fs_vec_l2norm(reinterpret_cast<fs_vec>(x), &xn));
-	memset(info, 0, sizeof(*info));
-	info->rhs_norm = (float)h.rhs_norm;
-	info->sol_norm_initial = zg ? 0.f : (float)h.sol0;
-	info->res_norm_initial = (float)h.res0;
-	info->res_norm_final = (float)h.res;
-	info->sol_norm_final = (float)xn;
-	info->restarts = h.restarts;
-	if (user_stop) {
-		info->status = FS_CONVERGED_USER;
-		info->iters = user_stop;
-	}
-	else {
-		info->status = h.status;
-		info->iters = h.info_iters;
-		if (h.res0 >= h.tol && info->iters == 0)
-			info->status = FS_DIVERGED_ITERS;  // gmres.hh:237-238
-	}
-	if (h.flags & KF_NONFINITE)
-		return set_err(ctx, FS_ERR_NON_FINITE, "GMRES: non-finite residual norm");
-	return FS_OK;
+	return gmres_info(s, zg, mixed, user_stop, xn, info);
 }
 
 }  // namespace

@@ -29,8 +29,10 @@
 //   pass 5: q_k = (u_k - Q s) / r over column k, and the next candidate
 //           u_{k+1} = (w - Q t - tau q_k) / r into column k + 1;
 //   pass 6: at the end of a cycle, s = Q^T u_m and alpha finish column m - 1.
-// Step 0 starts from the normalised q_0 (r = 1, no s).  The convergence test
-// of column k - 1 runs in step k's pass 4, one SpMV later than in CGS2.
+// Step 0 starts from the normalised q_0 (r = 1, no s).  The rotations and the
+// convergence test of column k - 1, which nothing in the step waits for, run
+// in a warp of their own beside step k's pass 5 (it writes columns k and
+// k + 1 only, which a solution of k columns does not read).
 //
 // Data movement.  Each pass streams tiles of v and of every basis vector into
 // a ring of shared-memory stages, issued by one producer lane as soon as the
@@ -65,6 +67,9 @@ constexpr int kOT = 256;                 // 8-byte elements per tile, one per co
 constexpr int kOCons = kOT / 32;         // consumer warps
 constexpr int kOThreads = kOT + 32;      // plus the producer warp
 constexpr int kOWarps = kOThreads / 32;
+// pass 5 has one more warp, which finishes the last Hessenberg column
+template<int PASS>
+constexpr int kOBlock = kOThreads + (PASS == 5 ? 32 : 0);
 constexpr int kOMaxStages = 32;
 constexpr int kStagedMax = 31;           // basis vectors the staged passes take
 constexpr int kOSlot = kOT * 8;          // bytes of one vector's tile
@@ -145,30 +150,65 @@ struct Elem<double> {
 	}
 };
 
-// per-CTA sums of the first nv of NV per-thread values -> part[b * nv + j]
-template<int NV>
-__device__ __forceinline__ void staged_block_sum(const double (&vals)[NV], int nv, double *part,
-                                                 double *sh) {
+// The CTA's sum of M elements in shared memory (16-byte aligned), by one
+// warp, in every lane: fixed point (resident.cuh), at least as accurate as a
+// tree of FP64 adds.
+template<int M>
+__device__ __forceinline__ double staged_sum(const float2 *p) {
+	const float4 *q = reinterpret_cast<const float4 *>(p);
+	double t = 0.0;
+#pragma unroll
+	for (int h = 0; h < M / 128; ++h) {
+		const float4 x = q[64 * h + (threadIdx.x & 31)], y = q[64 * h + 32 + (threadIdx.x & 31)];
+		const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+		const double u = res_warp_sum<8>(v);
+		t = h ? t + u : u;
+	}
+	return t;
+}
+template<int M>
+__device__ __forceinline__ double staged_sum(const double *p) {
+	double v[M / 32];
+#pragma unroll
+	for (int h = 0; h < M / 32; ++h)
+		v[h] = p[32 * h + (threadIdx.x & 31)];
+	return res_warp_sum<M / 32>(v);
+}
+
+// The CTA's sums of the consumers' accumulators -> part[b * nv + j].  Every
+// accumulator goes to shared memory (over the ring, which is drained), and
+// each warp sums whole values: nv values cost nv / 9 sums a warp instead of
+// nv shuffle trees in every warp, whose FP64 adds take 19 cycles an SM each
+// (62 values of pass 4: 9 x 310 adds, 26 us of the 101 us that the pass took
+// at kp1 = 31).  HALF: the consumers' halves hold different values, part 0
+// and part 1 (nv values each).  Every thread of the CTA calls it.
+template<class E, int NA, bool HALF>
+__device__ __forceinline__ void staged_block_sum(const E (&acc)[NA], int nv, double *part0,
+                                                 double *part1, unsigned char *scratch) {
+	E *s = reinterpret_cast<E *>(scratch);
 	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+	__syncthreads();  // the last tiles are read
+	if ((int)threadIdx.x < kOT) {
 #pragma unroll
-	for (int j = 0; j < NV; ++j) {
-		if (j < nv) {
-			double v = vals[j];
-#pragma unroll
-			for (int o = 16; o > 0; o >>= 1)
-				v += __shfl_down_sync(0xffffffffu, v, o);
+		for (int j = 0; j < NA; ++j)
+			if (j < nv)
+				s[j * kOT + threadIdx.x] = acc[j];
+	}
+	__syncthreads();
+	for (int v = wid; v < (HALF ? 2 * nv : nv); v += kOWarps) {
+		if constexpr (HALF) {
+			const int j = v < nv ? v : v - nv;
+			const double t = staged_sum<kOT / 2>(s + j * kOT + (v < nv ? 0 : kOT / 2));
 			if (lane == 0)
-				sh[j * kOWarps + wid] = v;
+				(v < nv ? part0 : part1)[(size_t)blockIdx.x * nv + j] = t;
+		}
+		else {
+			const double t = staged_sum<kOT>(s + v * kOT);
+			if (lane == 0)
+				part0[(size_t)blockIdx.x * nv + v] = t;
 		}
 	}
 	__syncthreads();
-	if ((int)threadIdx.x < nv) {
-		double t = 0.0;
-#pragma unroll
-		for (int w = 0; w < kOWarps; ++w)
-			t += sh[threadIdx.x * kOWarps + w];
-		part[(size_t)blockIdx.x * nv + threadIdx.x] = t;
-	}
 }
 
 // last CTA: out[j] = sum over CTAs of part[b * nv + j], j < nv <= 32.  Warp
@@ -205,7 +245,7 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
 }
 
 template<class T, int NA, int PASS>
-__global__ void __launch_bounds__(kOThreads, 1)
+__global__ void __launch_bounds__(kOBlock<PASS>, 1)
 k_gm_staged(OrthoArgs<T> a, const __grid_constant__ BasisMaps maps) {
 	static_assert(NA % 8 == 0 && NA <= 32, "accumulator slots");
 	using EL = Elem<T>;
@@ -220,9 +260,17 @@ k_gm_staged(OrthoArgs<T> a, const __grid_constant__ BasisMaps maps) {
 	__shared__ double sh[32 * kOWarps];
 	__shared__ double folded[64];
 	__shared__ int abort_flag;
-	if (stopped(a.st))
-		return;
+	__shared__ int stop_flag;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	pdl_wait();
+	pdl_trigger();
+	// one look a CTA: CTA 0's last warp may stop the solve during pass 5 (what
+	// the CTAs that still run it write is then not read again)
+	if (tid == 0)
+		stop_flag = stopped(a.st);
+	__syncthreads();
+	if (stop_flag)
+		return;
 	const int kp1 = a.kp1, S = a.stages;
 	const int64_t nelem = (a.n + R - 1) / R;
 	const int64_t ntile = (nelem + kOT - 1) / kOT;
@@ -304,7 +352,7 @@ k_gm_staged(OrthoArgs<T> a, const __grid_constant__ BasisMaps maps) {
 				mbar_wait(&full[j % S], (unsigned)((j / S) & 1));
 		}
 	}
-	else {
+	else if (warp < kOCons) {
 		const T inv = (T)(vn != 0.0 ? 1.0 / vn : 1.0);
 		for (int i = 0; i < nt; ++i) {
 			const int s = i % S;
@@ -388,69 +436,96 @@ k_gm_staged(OrthoArgs<T> a, const __grid_constant__ BasisMaps maps) {
 				break;
 		}
 	}
+	if constexpr (PASS == 5) {
+		// the rotations, the estimate and the stop test of column k - 1,
+		// which pass 4 finished, by a warp of its own beside the update
+		if (warp == kOWarps && blockIdx.x == 0 && kp1 > 1)
+			finish_step_warp(a.g, a.st, a.hist, sh);
+	}
 	if constexpr (PASS == 4 || PASS == 6) {
 		// pass 4: t and gamma (kp1 values, the first half of the consumers),
 		// then s and alpha (kp1 values, the second half) in a second block of
 		// partials; pass 6: s and alpha
-		const int grp = tid / (kOT / 2);
-		double vals[NA];
-#pragma unroll
-		for (int j = 0; j < NA; ++j)
-			vals[j] = j < kp1 && (PASS == 6 || grp == 0) ? EL::sum(acc[j]) : 0.0;
-		staged_block_sum<NA>(vals, kp1, a.part, sh);
 		double *part2 = a.part + (size_t)gridDim.x * kp1;
-		if constexpr (PASS == 4) {
-#pragma unroll
-			for (int j = 0; j < NA; ++j)
-				vals[j] = j < kp1 && grp == 1 ? EL::sum(acc[j]) : 0.0;
-			__syncthreads();  // sh of the first sum is read
-			staged_block_sum<NA>(vals, kp1, part2, sh);
-		}
+		staged_block_sum<E, NA, PASS == 4>(acc, kp1, a.part, part2, smem_raw);
 		if (last_block(a.counter)) {
+			GmState *g = a.g;
+			const int k = kp1 - 1, ldh = g->ld;
+			double *Hs = reinterpret_cast<double *>(smem_raw);  // H before the rotations, k columns
+			if constexpr (PASS == 4) {
+				for (int i = tid; i < kGmDelayedCols * k; i += blockDim.x)
+					Hs[i] = g->Hr[i];
+			}
 			staged_fold(a.part, kp1, folded, sh);
 			if constexpr (PASS == 4)
 				staged_fold(part2, kp1, folded + 32, sh);
-			// the scalar work, spread over the CTA where it is independent:
-			// every thread forms r and tau from shared memory; thread j
-			// finishes H(j, k - 1), thread i forms the tentative H(i, k)
-			GmState *g = a.g;
-			const int k = kp1 - 1, ldh = g->ld;
 			const double *s = PASS == 4 ? folded + 32 : folded;
 			const double *t = folded;
-			double ss = 0.0, st_ = 0.0;
-			for (int j = 0; j < k; ++j) {
-				ss += s[j] * s[j];
-				if constexpr (PASS == 4)
-					st_ += s[j] * t[j];
+			// s's and s't, a warp each
+			__shared__ double dots[3];
+			if (warp < 2) {
+				double d = 0.0;
+				if (lane < k)
+					d = s[lane] * (warp == 0 || PASS == 6 ? s[lane] : t[lane]);
+#pragma unroll
+				for (int o = 16; o > 0; o >>= 1)
+					d += __shfl_xor_sync(0xffffffffu, d, o);
+				if (lane == 0)
+					dots[warp] = d;
 			}
-			const double r = k > 0 ? sqrt(fmax(s[k] - ss, 0.0)) : 1.0;
-			const double rinv = r != 0.0 ? 1.0 / r : 1.0;
+			__syncthreads();
+			if (warp == 0) {
+				const double r = k > 0 ? sqrt(fmax(s[k] - dots[0], 0.0)) : 1.0;
+				const double rinv = r != 0.0 ? 1.0 / r : 1.0;
+				if (lane == 0) {
+					dots[0] = r;
+					dots[1] = PASS == 4 ? (t[k] - dots[1]) * rinv : 0.0;
+					dots[2] = rinv;
+				}
+			}
+			__syncthreads();
+			const double r = dots[0], rinv = dots[2];
 			if (k > 0) {
 				// column k - 1 is final: its tentative entries + s, r below
 				const int c = k - 1;
 				if (tid < k) {
-					const double hv = g->Hr[tid + kGmDelayedCols * c] + s[tid];
+					const double hv = (PASS == 4 ? Hs[tid + kGmDelayedCols * c]
+					                             : g->Hr[tid + kGmDelayedCols * c]) + s[tid];
 					g->Hr[tid + kGmDelayedCols * c] = hv;
 					g->H[tid + ldh * c] = hv;
+					if constexpr (PASS == 4)
+						Hs[tid + kGmDelayedCols * c] = hv;
 				}
 				if (tid == 0) {
 					g->Hr[k + kGmDelayedCols * c] = r;
 					g->H[k + ldh * c] = r;
 					g->vnorm = r;
+					if constexpr (PASS == 4)
+						Hs[k + kGmDelayedCols * c] = r;
 				}
 				__syncthreads();
-				finish_step_cta(g, a.st, a.hist, sh);
+				if constexpr (PASS == 6) {
+					if (warp == 0)
+						finish_step_warp(g, a.st, a.hist, sh);
+				}
 			}
 			if constexpr (PASS == 4) {
-				const double tau_k = (t[k] - st_) * rinv;
-				// tentative column k: ([t; tau] - H s) / r over rows 0..k
+				const double tau_k = dots[1];
+				// tentative column k: ([t; tau] - H s) / r over rows 0..k: row
+				// i in lane i, the k products split over the warps
+				double d = 0.0;
+				if (lane <= k)
+					for (int j = warp; j < k; j += kOWarps)
+						if (j + 1 >= lane)
+							d = ::fma(Hs[lane + kGmDelayedCols * j], s[j], d);
+				sh[warp * 32 + lane] = d;
+				__syncthreads();
 				if (tid <= k) {
-					const int i = tid;
-					double hs_i = 0.0;
-#pragma unroll 8
-					for (int j = i > 0 ? i - 1 : 0; j < k; ++j)
-						hs_i += g->Hr[i + kGmDelayedCols * j] * s[j];
-					g->Hr[i + kGmDelayedCols * k] = ((i < k ? t[i] : tau_k) - hs_i) * rinv;
+					double hs_i = sh[tid];
+#pragma unroll
+					for (int w = 1; w < kOWarps; ++w)
+						hs_i += sh[w * 32 + tid];
+					g->Hr[tid + kGmDelayedCols * k] = ((tid < k ? t[tid] : tau_k) - hs_i) * rinv;
 				}
 				if (tid < k) {
 					g->h1[tid] = s[tid];
@@ -468,14 +543,12 @@ k_gm_staged(OrthoArgs<T> a, const __grid_constant__ BasisMaps maps) {
 	if constexpr (PASS == 1 || PASS == 2) {
 		// pass 2 puts ||v'||^2 right after the kp1 dots
 		constexpr int NS = PASS == 2 ? NA + 1 : NA;
-		double vals[NS];
+		E vals[NS];
 #pragma unroll
-		for (int j = 0; j < NS; ++j) {
-			const double aj = j < NA ? EL::sum(acc[j < NA ? j : 0]) : 0.0;
-			vals[j] = j < kp1 ? aj : (PASS == 2 && j == kp1 ? EL::sum(accn) : 0.0);
-		}
+		for (int j = 0; j < NS; ++j)
+			vals[j] = j < kp1 ? acc[j < NA ? j : 0] : accn;
 		const int nv = PASS == 2 ? kp1 + 1 : kp1;
-		staged_block_sum<NS>(vals, nv, a.part, sh);
+		staged_block_sum<E, NS, false>(vals, nv, a.part, nullptr, smem_raw);
 		if (last_block(a.counter)) {
 			staged_fold(a.part, nv, folded, sh);
 			GmState *g = a.g;
@@ -498,7 +571,8 @@ k_gm_staged(OrthoArgs<T> a, const __grid_constant__ BasisMaps maps) {
 					g->vnorm = vn2;
 				}
 				__syncthreads();
-				finish_step_cta(g, a.st, a.hist, sh);
+				if (warp == 0)
+					finish_step_warp(g, a.st, a.hist, sh);
 			}
 			if (tid == 0)
 				*a.counter = 0;
@@ -518,8 +592,8 @@ int launch_staged(Ctx *ctx, const OrthoArgs<T> &a, const BasisMaps &maps) {
 			               kOSmemBudget + 128);
 		ready = true;
 	}
-	kern<<<ctx->sms, kOThreads, smem, ctx->stream>>>(a, maps);
-	return check_launch(ctx, "gmres staged orthogonalisation");
+	return check_launch_rc(ctx, launch_pdl(ctx->stream, kern, ctx->sms, kOBlock<PASS>, smem, a, maps),
+	                       "gmres staged orthogonalisation");
 }
 
 template<class T, int PASS>

@@ -10,11 +10,8 @@
 // takes; the two reductions take 6,500 each with the CTAs' skew, the scalars
 // 3,100.  At 128^2 (128 rows) the reductions take 3,700 each, the SpMV 1,900
 // (mostly the packets' latency), the scalars 2,500, update and direction 1,600.
-#include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <map>
-#include <mutex>
 
 #include "resident.cuh"
 
@@ -37,29 +34,6 @@ struct ResCg {
 	int rows;                 // rows per CTA
 	int smem;                 // dynamic shared memory, bytes
 };
-
-// own rows l = tid, tid + nt, ...: U at a time while there are U, all of
-// load(l) before any store(l, value), then one by one
-template<int U, class L, class S>
-__device__ __forceinline__ void res_rows(int cnt, L &&load, S &&store) {
-	using T = decltype(load(0));
-	const int nt = (int)blockDim.x;
-	int l = (int)threadIdx.x;
-	if constexpr (U > 1)
-		for (; l + (U - 1) * nt < cnt; l += U * nt) {
-			T t[U];
-#pragma unroll
-			for (int u = 0; u < U; ++u)
-				t[u] = load(l + u * nt);
-#pragma unroll
-			for (int u = 0; u < U; ++u)
-				store(l + u * nt, t[u]);
-		}
-	for (; l < cnt; l += nt) {
-		const T t = load(l);
-		store(l, t);
-	}
-}
 
 // PKT: the slice's p fits in shared memory and the other slices read it as
 // packets; otherwise p is a global vector and the direction step ends with a
@@ -310,71 +284,6 @@ k_cg_resident(ResCg a) {
 	tm.finish();
 }
 
-struct ResShape {
-	int grid, threads, rows, smem;
-};
-
-// One CTA per SM, at least kMinRows rows each (a CTA's share of a grid_sum
-// costs the same however few rows it holds); a thread per row up to
-// kResThreads, four warps at least (one per value of a grid_sum); `per_row`
-// bytes of shared memory a row, as far as they go.
-ResShape res_shape(Ctx *ctx, int64_t n, int per_row, int smem_max) {
-	constexpr int kMinRows = 64;
-	const int64_t cap = std::min(ctx->sms, kResMaxG);
-	int64_t g = std::max<int64_t>(1, std::min(cap, (n + kMinRows - 1) / kMinRows));
-	int64_t rows = ((n + g - 1) / g + 31) / 32 * 32;
-	g = (n + rows - 1) / rows;
-	ResShape s;
-	s.grid = (int)g;
-	s.rows = (int)rows;
-	s.threads = (int)std::min<int64_t>(kResThreads, std::max<int64_t>(128, rows));
-	// (count * 8 + 15) & ~15 per array: rows is a multiple of 32
-	s.smem = (int)std::min<int64_t>(smem_max, rows * per_row);
-	return s;
-}
-
-template<class Args>
-int res_launch(Ctx *ctx, void (*kern)(Args), const ResShape &sh, const Args &a, const char *what) {
-	cudaLaunchConfig_t cfg{};
-	cfg.gridDim = dim3((unsigned)sh.grid);
-	cfg.blockDim = dim3((unsigned)sh.threads);
-	cfg.dynamicSmemBytes = (size_t)sh.smem;
-	cfg.stream = ctx->stream;
-	cudaLaunchAttribute at[1];
-	at[0].id = cudaLaunchAttributeCooperative;
-	at[0].val.cooperative = 1;
-	cfg.attrs = at;
-	cfg.numAttrs = 1;
-	return check_launch_rc(ctx, cudaLaunchKernelEx(&cfg, kern, a), what);
-}
-
-// dynamic shared memory a resident kernel may use (its static part is taken
-// off), set on the kernel once per device; 0 when the device refuses it
-template<class Args>
-int res_smem_max(Ctx *ctx, void (*kern)(Args)) {
-	static std::map<std::pair<int, const void *>, int> known;
-	static std::mutex mu;
-	std::lock_guard<std::mutex> lock(mu);
-	const auto key = std::make_pair(ctx->device, (const void *)kern);
-	const auto it = known.find(key);
-	if (it != known.end())
-		return it->second;
-	int optin = 0;
-	cudaFuncAttributes fa;
-	if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) !=
-	        cudaSuccess ||
-	    cudaFuncGetAttributes(&fa, kern) != cudaSuccess)
-		return 0;
-	int bytes = std::max(0, (optin - (int)fa.sharedSizeBytes) / 1024 * 1024);
-	if (bytes > 0 &&
-	    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
-		cudaGetLastError();
-		bytes = 0;
-	}
-	known.emplace(key, bytes);
-	return bytes;
-}
-
 // Rows up to which FP64 CG runs resident.  The gain falls from the launches'
 // share of an iteration to the little that the vectors kept in shared memory
 // save (us per iteration, kernel per phase -> resident): 18.5 -> 6.5 at 32^2,
@@ -389,39 +298,15 @@ constexpr int kResPktArrays = 4;
 
 }  // namespace
 
-// The operator as a grid stencil in the storage that the FP64 SpMV would use;
-// false when it is none
-static bool res_grid64(const Csr *A, ResGrid<double> &g, bool &gen) {
-	if (stores_no_rows(A) || A->view || A->grid_nx <= 0 || A->coding != kCodingGrid)
-		return false;
-	if (A->sym64_valid)
-		gen = false;
-	else if (A->gen64_valid)
-		gen = true;
-	else
-		return false;
-	g.S = gen ? A->gen64 : A->sym64;
-	g.ld = A->sym_ld;
-	g.n = (int)A->nrows;
-	g.nx = A->grid_nx;
-	g.ny = A->grid_ny;
-	g.nz = A->grid_nz;
-	return true;
-}
-
-int ensure_res_slots(Solver *s);
-
 // FP64 CG; `taken` = 0 when the solve is not one for the resident kernel
 int cg_apply_resident(Solver *s, Vec *b, Vec *x, fs_solve_info *info, int *taken) {
 	*taken = 0;
 	Ctx *ctx = s->ctx;
 	ResCg a{};
 	bool gen = false;
-	if (s->diag || s->n > kResCgRows || !res_grid64(s->A, a.A, gen))
+	if (s->diag || s->n > kResCgRows || !res_grid<double>(s->A, a.A, gen))
 		return FS_OK;
 	const int K = s->A->nsym;
-	if (K < 1 || K > 3)
-		return FS_OK;
 	// mask, p, r, w, x, dinv and the diagonals, as far as they fit
 	const int per_row = 1 + 8 * (5 + 1 + (gen ? 2 * K : K));
 	using Kern = void (*)(ResCg);
@@ -439,14 +324,7 @@ int cg_apply_resident(Solver *s, Vec *b, Vec *x, fs_solve_info *info, int *taken
 	const bool pkt = (int64_t)sh.rows * (1 + 8 * kResPktArrays) <= smem_max;
 	const Kern kern = kerns[gen][pkt][K - 1];
 	if (pkt) {
-		if (!s->res_pk) {
-			void *q = nullptr;
-			const size_t bytes = (size_t)s->n * sizeof(ulonglong2);
-			FS_CUDA_TRY(ctx, cudaMalloc(&q, bytes));
-			s->bufs.push_back(q);
-			FS_CUDA_TRY(ctx, cudaMemsetAsync(q, 0, bytes, ctx->stream));
-			s->res_pk = (ulonglong2 *)q;
-		}
+		FS_TRY(ensure_res_packets(s));
 		a.pk = s->res_pk;
 	}
 	FS_TRY(ensure_res_slots(s));
@@ -497,6 +375,18 @@ int ensure_res_slots(Solver *s) {
 	FS_CUDA_TRY(s->ctx, cudaMemsetAsync(p, 0, sizeof(ResSlots), s->ctx->stream));
 	FS_CUDA_TRY(s->ctx, cudaMemsetAsync(&((ResSlots *)p)->epoch, 1, 1, s->ctx->stream));
 	s->res_slots = (ResSlots *)p;
+	return FS_OK;
+}
+
+int ensure_res_packets(Solver *s) {
+	if (s->res_pk)
+		return FS_OK;
+	void *p = nullptr;
+	const size_t bytes = (size_t)s->n * sizeof(ulonglong2);
+	FS_CUDA_TRY(s->ctx, cudaMalloc(&p, bytes));
+	s->bufs.push_back(p);
+	FS_CUDA_TRY(s->ctx, cudaMemsetAsync(p, 0, bytes, s->ctx->stream));
+	s->res_pk = (ulonglong2 *)p;
 	return FS_OK;
 }
 

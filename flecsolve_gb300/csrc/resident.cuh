@@ -25,6 +25,10 @@
 // word and leaves, as do the others when their own waits run out.
 #pragma once
 
+#include <algorithm>
+#include <map>
+#include <mutex>
+
 #include "solver.cuh"
 
 namespace fsg {
@@ -138,8 +142,85 @@ __device__ __forceinline__ ResFix res_fix_cta(ResFix f) {
 	return {hi * (1 << 13) + ((lo + (1ll << 32)) >> 33), E};
 }
 
+// (hi 2^16 + lo 2^-30) 2^(E - 1075)
+__device__ __forceinline__ double res_fix_double(long long hi, long long lo, int E) {
+	const double t = fma((double)lo, 0x1p-46, (double)hi);
+	const int k = E - 1059;
+	if (k >= -1022)
+		return t * __longlong_as_double((long long)(k + 1023) << 52);
+	return t * 0x1p-600 * __longlong_as_double((long long)(k + 600 + 1023) << 52);
+}
+
+// the sum of N doubles a lane over a warp, in every lane
+template<int N>
+__device__ __forceinline__ double res_warp_sum(const double (&v)[N]) {
+	int E = 1;
+#pragma unroll
+	for (int i = 0; i < N; ++i)
+		E = max(E, (int)((unsigned long long)__double_as_longlong(v[i]) >> 52) & 0x7ff);
+	E = __reduce_max_sync(0xffffffffu, E);
+	if (E == 0x7ff) {
+		// not finite: the plain sum has the right infinity or NaN
+		double t = 0.0;
+#pragma unroll
+		for (int i = 0; i < N; ++i)
+			t += v[i];
+		for (int o = 16; o > 0; o >>= 1)
+			t += __shfl_xor_sync(0xffffffffu, t, o);
+		return t;
+	}
+	ResPieces s;
+	s.clear();
+#pragma unroll
+	for (int i = 0; i < N; ++i) {
+		const unsigned long long b = (unsigned long long)__double_as_longlong(v[i]);
+		const int e = (int)(b >> 52) & 0x7ff;
+		s.add((b & ((1ull << 52) - 1)) | (e ? 1ull << 52 : 0ull), E - max(e, 1), b >> 63);
+	}
+	s.warp_sum();
+	long long hi, lo;
+	s.split(hi, lo);
+	return res_fix_double(hi, lo, E);
+}
+
+// the sum of N <= 8 floats a lane over a warp, in every lane: the 24-bit
+// mantissas at the largest exponent of the warp with 31 bits below its unit,
+// added in 64-bit integers and rounded once
+template<int N>
+__device__ __forceinline__ double res_warp_sum(const float (&v)[N]) {
+	static_assert(N <= 8, "24 + 31 bits, 8 a lane, 32 lanes: below 2^63");
+	int E = 1;
+#pragma unroll
+	for (int i = 0; i < N; ++i)
+		E = max(E, (__float_as_int(v[i]) >> 23) & 0xff);
+	E = __reduce_max_sync(0xffffffffu, E);
+	if (E == 0xff) {
+		double t = 0.0;
+#pragma unroll
+		for (int i = 0; i < N; ++i)
+			t += (double)v[i];
+		for (int o = 16; o > 0; o >>= 1)
+			t += __shfl_xor_sync(0xffffffffu, t, o);
+		return t;
+	}
+	long long q = 0;
+#pragma unroll
+	for (int i = 0; i < N; ++i) {
+		const int b = __float_as_int(v[i]), e = (b >> 23) & 0xff;
+		const int m = (b & 0x7fffff) | (e ? 0x800000 : 0);
+		const int d = min(E - max(e, 1), 63);
+		q += ((long long)(b < 0 ? -m : m) << 31) >> d;
+	}
+	constexpr long long M = (1ll << 26) - 1;
+	const long long p0 = __reduce_add_sync(0xffffffffu, (int)(q & M));
+	const long long p1 = __reduce_add_sync(0xffffffffu, (int)(q >> 26 & M));
+	const long long p2 = __reduce_add_sync(0xffffffffu, (int)(q >> 52));
+	return (double)(p2 * (1ll << 52) + p1 * (1ll << 26) + p0) *
+	       __longlong_as_double((long long)(E - 181 + 1023) << 52);
+}
+
 // the sum of the CTAs' sums, Q a lane, as a double (the same in every lane)
-template<int Q>
+template<int Q, int F = 0>
 __device__ __forceinline__ double res_fix_grid(const ResFix (&f)[Q]) {
 	int E = 1;
 #pragma unroll
@@ -164,12 +245,38 @@ __device__ __forceinline__ double res_fix_grid(const ResFix (&f)[Q]) {
 	s.warp_sum();
 	long long hi, lo;
 	s.split(hi, lo);
-	// (hi + lo 2^-46) 2^(E - 1059)
-	const double t = fma((double)lo, 0x1p-46, (double)hi);
-	const int k = E - 1059;
-	if (k >= -1022)
-		return t * __longlong_as_double((long long)(k + 1023) << 52);
-	return t * 0x1p-600 * __longlong_as_double((long long)(k + 600 + 1023) << 52);
+	return res_fix_double(hi, lo, E - F);
+}
+
+// the sum of 8 floats a lane over a warp, F = 3 (29 bits below the unit of
+// the largest: 24 + 29 + 8 bits, below 2^62)
+__device__ __forceinline__ ResFix res_fix_warp8(const float (&v)[8]) {
+	int E = 1;
+#pragma unroll
+	for (int i = 0; i < 8; ++i)
+		E = max(E, (__float_as_int(v[i]) >> 23) & 0xff);
+	E = __reduce_max_sync(0xffffffffu, E);
+	if (E == 0xff) {
+		int cls = 0;
+#pragma unroll
+		for (int i = 0; i < 8; ++i)
+			cls |= isnan(v[i]) ? 4 : isinf(v[i]) ? (v[i] < 0.f ? 2 : 1) : 0;
+		return res_special(cls);
+	}
+	long long q = 0;
+#pragma unroll
+	for (int i = 0; i < 8; ++i) {
+		const int b = __float_as_int(v[i]), e = (b >> 23) & 0xff;
+		const int m = (b & 0x7fffff) | (e ? 0x800000 : 0);
+		const int d = min(E - max(e, 1), 63);
+		q += ((long long)(b < 0 ? -m : m) << 29) >> d;
+	}
+	constexpr long long M = (1ll << 26) - 1;
+	const long long p0 = __reduce_add_sync(0xffffffffu, (int)(q & M));
+	const long long p1 = __reduce_add_sync(0xffffffffu, (int)(q >> 26 & M));
+	const long long p2 = __reduce_add_sync(0xffffffffu, (int)(q >> 52));
+	// q 2^(E - 179) = q 2^(e - 1075 - 3)
+	return {p2 * (1ll << 52) + p1 * (1ll << 26) + p0, E + 899};
 }
 
 // ------------------------------------------------------------ messages --
@@ -241,6 +348,34 @@ struct ResTeam {
 		*(volatile int *)&sh->fail = 1;
 	}
 
+	// One warp: the grid's messages of this epoch, one slot a CTA ({0, 1} past
+	// the grid); false in every lane when one did not arrive
+	__device__ bool gather(const ulonglong2 *set, ResFix (&f)[kResMaxG / 32]) {
+		constexpr int Q = kResMaxG / 32;
+		const int lane = threadIdx.x & 31, G = (int)gridDim.x;
+		bool here = false;
+		for (int it = 0; !here && it < kResPolls; ++it) {
+			// every slot of this lane in flight, then the tags
+			ulonglong2 m[Q];
+#pragma unroll
+			for (int q = 0; q < Q; ++q)
+				if (q * 32 < G)
+					m[q] = res_ld16(&set[min(q * 32 + lane, G - 1)]);
+			here = true;
+#pragma unroll
+			for (int q = 0; q < Q; ++q)
+				if (q * 32 < G) {
+					here = here && m[q].y >> 16 == epoch;
+					f[q] = {(long long)m[q].x, (int)(m[q].y & 0xffff)};
+				}
+		}
+#pragma unroll
+		for (int q = 0; q < Q; ++q)
+			if (q * 32 + lane >= G)
+				f[q] = {0, 1};
+		return __all_sync(0xffffffffu, here);
+	}
+
 	// Sums NV values over the grid.  Every thread calls it; warp k carries
 	// value k through the messages (in parallel: two values take a third
 	// longer than one) and has its total in every lane of the returned
@@ -272,32 +407,10 @@ struct ResTeam {
 			res_xchg16(&set[blockIdx.x], (unsigned long long)own.q,
 			           epoch << 16 | (unsigned long long)own.e);
 		res_hold(clock64());
-		constexpr int Q = kResMaxG / 32;
-		const int G = (int)gridDim.x;
-		ResFix f[Q];
-		bool here = false;
-		for (int it = 0; !here && it < kResPolls; ++it) {
-			// every slot of this lane in flight, then the tags
-			ulonglong2 m[Q];
-#pragma unroll
-			for (int q = 0; q < Q; ++q)
-				if (q * 32 < G)
-					m[q] = res_ld16(&set[min(q * 32 + lane, G - 1)]);
-			here = true;
-#pragma unroll
-			for (int q = 0; q < Q; ++q)
-				if (q * 32 < G) {
-					here = here && m[q].y >> 16 == epoch;
-					f[q] = {(long long)m[q].x, (int)(m[q].y & 0xffff)};
-				}
-		}
-#pragma unroll
-		for (int q = 0; q < Q; ++q)
-			if (q * 32 + lane >= G)
-				f[q] = {0, 1};
-		if (!__all_sync(0xffffffffu, here) && lane == 0)
+		ResFix f[kResMaxG / 32];
+		if (!gather(set, f) && lane == 0)
 			failed();
-		const double t = res_fix_grid<Q>(f);
+		const double t = res_fix_grid<kResMaxG / 32>(f);
 		if (PUB)
 			__threadfence();
 		return t;
@@ -345,6 +458,33 @@ __device__ __forceinline__ double res_quotient(double a, double b, double y) {
 	const bool safe = m > 0x1p-900 && m < 0x1p900 && n > 0x1p-900 && n < 0x1p900 && fabs(q) > 0x1p-900 &&
 	                  fabs(q) < 0x1p900;
 	return safe ? r : a / b;
+}
+
+// the payload of a packet that had not arrived at the first look (its own
+// function: inlined, the loops of a row's neighbours cost the caller spills)
+static __device__ __noinline__ unsigned long long res_await(const ulonglong2 *p, unsigned long long tag,
+                                                     ResShared *sh, unsigned *err) {
+	for (int it = 0; it < kResPolls && !*(volatile int *)&sh->fail; ++it) {
+		const ulonglong2 m = res_ld16(p);
+		if (m.y == tag)
+			return m.x;
+	}
+	atomicOr(err, 0x40u);
+	*(volatile int *)&sh->fail = 1;
+	return 0;
+}
+
+// a vector entry's packet payload
+__device__ __forceinline__ unsigned long long res_pack(double v) {
+	return (unsigned long long)__double_as_longlong(v);
+}
+__device__ __forceinline__ unsigned long long res_pack(float v) { return __float_as_uint(v); }
+template<class V>
+__device__ __forceinline__ V res_unpack(unsigned long long b) {
+	if constexpr (sizeof(V) == 8)
+		return __longlong_as_double((long long)b);
+	else
+		return __uint_as_float((unsigned)b);
 }
 
 // Grid-stencil operator of a resident kernel: the symmetric or the general
@@ -433,16 +573,10 @@ struct ResRows {
 #pragma unroll
 			for (int t = 0; t < 2 * K; ++t)
 				if (!in[t]) {
-					const int slot = t < K ? t : t + 1;
-					for (int it = 0; w[t].y != tag; ++it) {
-						if (it >= kResPolls || *(volatile int *)&tm.sh->fail) {
-							tm.failed();
-							break;
-						}
-						const int e = t < K ? K - 1 - t : t - K;
-						w[t] = res_ld16(pk + (lo + (t < K ? l - d[e] : l + d[e])));
-					}
-					x[slot] = (V)__longlong_as_double((long long)w[t].x);
+					const int slot = t < K ? t : t + 1, e = t < K ? K - 1 - t : t - K;
+					if (w[t].y != tag)
+						w[t].x = res_await(pk + (lo + (t < K ? l - d[e] : l + d[e])), tag, tm.sh, tm.err);
+					x[slot] = res_unpack<V>(w[t].x);
 				}
 		}
 		V s = V(0);
@@ -473,5 +607,125 @@ struct ResSmem {
 		return p;
 	}
 };
+
+// own rows l = tid, tid + nt, ...: U at a time while there are U, all of
+// load(l) before any store(l, value), then one by one
+template<int U, class L, class S>
+__device__ __forceinline__ void res_rows(int cnt, L &&load, S &&store) {
+	using T = decltype(load(0));
+	const int nt = (int)blockDim.x;
+	int l = (int)threadIdx.x;
+	if constexpr (U > 1)
+		for (; l + (U - 1) * nt < cnt; l += U * nt) {
+			T t[U];
+#pragma unroll
+			for (int u = 0; u < U; ++u)
+				t[u] = load(l + u * nt);
+#pragma unroll
+			for (int u = 0; u < U; ++u)
+				store(l + u * nt, t[u]);
+		}
+	for (; l < cnt; l += nt) {
+		const T t = load(l);
+		store(l, t);
+	}
+}
+
+// ---------------------------------------------------------------- host --
+
+struct ResShape {
+	int grid, threads, rows, smem;
+};
+
+// One CTA per SM, at least kMinRows rows each (a CTA's share of a grid_sum
+// costs the same however few rows it holds); a thread per row up to
+// kResThreads, four warps at least (one per value of a grid_sum); `per_row`
+// bytes of shared memory a row, as far as they go.
+inline ResShape res_shape(Ctx *ctx, int64_t n, int per_row, int smem_max) {
+	constexpr int kMinRows = 64;
+	const int64_t cap = std::min(ctx->sms, kResMaxG);
+	int64_t g = std::max<int64_t>(1, std::min(cap, (n + kMinRows - 1) / kMinRows));
+	int64_t rows = ((n + g - 1) / g + 31) / 32 * 32;
+	g = (n + rows - 1) / rows;
+	ResShape s;
+	s.grid = (int)g;
+	s.rows = (int)rows;
+	s.threads = (int)std::min<int64_t>(kResThreads, std::max<int64_t>(128, rows));
+	// (count * 8 + 15) & ~15 per array: rows is a multiple of 32
+	s.smem = (int)std::min<int64_t>(smem_max, rows * per_row);
+	return s;
+}
+
+template<class Args>
+inline int res_launch(Ctx *ctx, void (*kern)(Args), const ResShape &sh, const Args &a, const char *what) {
+	cudaLaunchConfig_t cfg{};
+	cfg.gridDim = dim3((unsigned)sh.grid);
+	cfg.blockDim = dim3((unsigned)sh.threads);
+	cfg.dynamicSmemBytes = (size_t)sh.smem;
+	cfg.stream = ctx->stream;
+	cudaLaunchAttribute at[1];
+	at[0].id = cudaLaunchAttributeCooperative;
+	at[0].val.cooperative = 1;
+	cfg.attrs = at;
+	cfg.numAttrs = 1;
+	return check_launch_rc(ctx, cudaLaunchKernelEx(&cfg, kern, a), what);
+}
+
+// dynamic shared memory a resident kernel may use (its static part is taken
+// off), set on the kernel once per device; 0 when the device refuses it
+template<class Args>
+inline int res_smem_max(Ctx *ctx, void (*kern)(Args)) {
+	static std::map<std::pair<int, const void *>, int> known;
+	static std::mutex mu;
+	std::lock_guard<std::mutex> lock(mu);
+	const auto key = std::make_pair(ctx->device, (const void *)kern);
+	const auto it = known.find(key);
+	if (it != known.end())
+		return it->second;
+	int optin = 0;
+	cudaFuncAttributes fa;
+	if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) !=
+	        cudaSuccess ||
+	    cudaFuncGetAttributes(&fa, kern) != cudaSuccess)
+		return 0;
+	int bytes = std::max(0, (optin - (int)fa.sharedSizeBytes) / 1024 * 1024);
+	if (bytes > 0 &&
+	    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+		cudaGetLastError();
+		bytes = 0;
+	}
+	known.emplace(key, bytes);
+	return bytes;
+}
+
+// The operator as a grid stencil in the storage that the SpMV on values of V
+// would use; false when it is none
+template<class V>
+inline bool res_grid(const Csr *A, ResGrid<V> &g, bool &gen) {
+	constexpr bool f32 = sizeof(V) == 4;
+	if (stores_no_rows(A) || A->view || A->grid_nx <= 0 || A->coding != kCodingGrid ||
+	    A->nsym < 1 || A->nsym > 3)
+		return false;
+	if (f32 ? A->sym32_valid : A->sym64_valid)
+		gen = false;
+	else if (f32 ? A->gen32_valid : A->gen64_valid)
+		gen = true;
+	else
+		return false;
+	if constexpr (f32)
+		g.S = gen ? A->gen32 : A->sym32;
+	else
+		g.S = gen ? A->gen64 : A->sym64;
+	g.ld = A->sym_ld;
+	g.n = (int)A->nrows;
+	g.nx = A->grid_nx;
+	g.ny = A->grid_ny;
+	g.nz = A->grid_nz;
+	return true;
+}
+
+// the solver's messages and row packets, allocated on first use (resident.cu)
+int ensure_res_slots(Solver *s);
+int ensure_res_packets(Solver *s);
 
 }  // namespace fsg
