@@ -871,6 +871,10 @@ int gmres_run(Solver *s, Vec *b, Vec *x, fs_solve_info *info, bool mixed) {
 			cudaGraphExecDestroy(kv.second.exec);
 		s->graphs.clear();
 	}
+	int taken = 0;
+	FS_TRY(gmres_apply_resident<T>(s, b, x, mdim, mixed, &taken));
+	if (taken)
+		return gmres_info(s, zg, mixed, 0, s->hst->aux[2], info);
 	{
 		// the staged CGS2 passes read the basis through a tensor map (encoded
 		// on the host, once per basis, type and shape); without one the

@@ -6,10 +6,11 @@
 //
 // Bound: the FP64 pipe issues a warp instruction per SM in 19 cycles, and an
 // iteration needs 14 per 32 rows (SpMV 7, p'Ap 1, update 5, direction 1).  At
-// 77^3 (3,008 rows a CTA) that is 25,000 of the 42,800 cycles an iteration
-// takes; the two reductions take 6,500 each with the CTAs' skew, the scalars
-// 3,100.  At 128^2 (128 rows) the reductions take 3,700 each, the SpMV 1,900
-// (mostly the packets' latency), the scalars 2,500, update and direction 1,600.
+// 77^3 (3,008 rows a CTA) that is 25,000 of the 39,000 cycles an iteration
+// takes; the reductions with the CTAs' skew and the scalars take the rest.  At
+// 128^2 (128 rows, 11,600 cycles) the two reductions take about 3,500 each, the
+// SpMV 1,500 (mostly the packets' latency), the scalars 2,000, update and
+// direction 1,500.
 #include <cmath>
 #include <cstring>
 
@@ -158,7 +159,7 @@ k_cg_resident(ResCg a) {
 	while (alive && !sh.stop) {
 		// w = A p, p'Ap -> alpha = rho / p'Ap (cg.hh:94-106)
 		double s1[1] = {0.0};
-		res_rows<PKT && K == 3 ? 1 : 2>(
+		res_rows<2>(
 			cnt, [&](int l) { return A.template sum<PKT>(l, pl, a.p, a.pk, tag, tm); },
 			[&](int l, double s) {
 				w[l] = s;
@@ -286,9 +287,9 @@ k_cg_resident(ResCg a) {
 
 // Rows up to which FP64 CG runs resident.  The gain falls from the launches'
 // share of an iteration to the little that the vectors kept in shared memory
-// save (us per iteration, kernel per phase -> resident): 18.5 -> 6.5 at 32^2,
-// 20.8 -> 6.5 at 128^2, 34.1 -> 12.8 at 512^2, 48 -> 20.7 at 77^3, 57.2 -> 33.6
-// at 96^3, 91.1 -> 65.0 at 128^3, 113.3 -> 93.8 at 144^3 (3.0 M rows).
+// save (us per iteration, kernel per phase -> resident): 18.5 -> 6.4 at 32^2,
+// 20.8 -> 5.6 at 128^2, 34.1 -> 12.8 at 512^2, 48 -> 18.8 at 77^3, 57.2 -> 30.5
+// at 96^3, 91.1 -> 63.8 at 128^3, 113.3 -> 93.8 at 144^3 (3.0 M rows).
 // Beyond, one CTA per SM no longer hides the memory that does not fit.
 constexpr int64_t kResCgRows = 3000000;
 // Packets are used while the slice's mask and p, r, w and x fit in its shared

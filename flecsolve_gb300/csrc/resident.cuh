@@ -529,64 +529,77 @@ struct ResRows {
 
 	// sum of the own row l over a vector whose own rows are vl (indexed from
 	// the slice's first row); rows of other slices come from packets `pk`
-	// carrying `tag` (PKT) or from the global vector vg
+	// carrying `tag` (PKT) or from the global vector vg.  The packets of the
+	// two outermost neighbours, which most rows of a 2-D or 3-D slice need, are
+	// in flight while the others are read; an inner neighbour is outside the
+	// slice only near its ends and is awaited where it is added.
 	template<bool PKT>
 	__device__ __forceinline__ V sum(int l, const V *vl, const V *vg, const ulonglong2 *pk,
 	                                 unsigned long long tag, ResTeam &tm) const {
 		const unsigned m = mask[l];
-		V c[2 * K + 1], x[2 * K + 1];
-		ulonglong2 w[2 * K];
-		bool in[2 * K];
-		auto at = [&](int t, int slot, int j) {
-			in[t] = (unsigned)j < (unsigned)cnt;
-			if constexpr (PKT) {
-				if (in[t])
-					x[slot] = vl[j];
-				else
-					w[t] = res_ld16(pk + (lo + j));
-			}
-			else {
-				const V *q = in[t] ? vl + j : vg + (lo + j);
-				x[slot] = *q;
-			}
-		};
-#pragma unroll
-		for (int t = 0; t < K; ++t) {
-			// lower neighbour of offset d[K - 1 - t], upper neighbour of d[t];
-			// an absent one reads the own row and its term is not added
-			const int e = K - 1 - t;
-			const bool lower = m >> (2 - e) & 1, upper = m >> (3 + t) & 1;
-			const int jl = lower ? l - d[e] : l, ju = upper ? l + d[t] : l;
-			at(t, t, jl);
-			at(K + t, K + 1 + t, ju);
-			if (GEN)
-				c[t] = L[e][l];
-			else {
-				const V *q = jl >= 0 ? U[e] + jl : G + ((int64_t)e * ld + lo + jl);
-				c[t] = *q;
-			}
-			c[K + 1 + t] = U[t][l];
-		}
-		x[K] = vl[l];
-		c[K] = D[l];
+		constexpr int O = K - 1;  // outermost dimension
+		const bool has_lo = m >> (2 - O) & 1, has_hi = m >> (3 + O) & 1;
+		// an absent neighbour reads the own row and its term is not added
+		const int jl = has_lo ? l - d[O] : l, jh = has_hi ? l + d[O] : l;
+		const bool in_lo = jl >= 0, in_hi = jh < cnt;
+		ulonglong2 wl, wh;
+		V xl, xh;
 		if constexpr (PKT) {
+			if (!in_lo)
+				wl = res_ld16(pk + (lo + jl));
+			if (!in_hi)
+				wh = res_ld16(pk + (lo + jh));
+		}
+		else {
+			xl = *(in_lo ? vl + jl : vg + (lo + jl));
+			xh = *(in_hi ? vl + jh : vg + (lo + jh));
+		}
+		auto lower = [&](int e, int j) -> V {  // a(l, l - d[e]), j = l - d[e]
+			if constexpr (GEN)
+				return L[e][l];
+			else
+				return *(j >= 0 ? U[e] + j : G + ((int64_t)e * ld + lo + j));
+		};
+		V x[2 * K + 1], c[2 * K + 1];  // inner neighbours and all coefficients
+		c[0] = lower(O, jl);
+		c[2 * K] = U[O][l];
 #pragma unroll
-			for (int t = 0; t < 2 * K; ++t)
-				if (!in[t]) {
-					const int slot = t < K ? t : t + 1, e = t < K ? K - 1 - t : t - K;
-					if (w[t].y != tag)
-						w[t].x = res_await(pk + (lo + (t < K ? l - d[e] : l + d[e])), tag, tm.sh, tm.err);
-					x[slot] = res_unpack<V>(w[t].x);
-				}
+		for (int t = 1; t < 2 * K; ++t) {
+			// t < K: lower neighbour of d[K - 1 - t]; t > K: upper of d[t - K - 1]
+			const int e = t < K ? K - 1 - t : t - K - 1;
+			const bool has = t == K || (t < K ? m >> (2 - e) & 1 : m >> (3 + e) & 1);
+			const int j = t == K || !has ? l : t < K ? l - d[e] : l + d[e];
+			const bool in = t == K || (t < K ? j >= 0 : j < cnt);
+			if constexpr (PKT) {
+				if (in)
+					x[t] = vl[j];
+				else
+					x[t] = res_unpack<V>(res_await(pk + (lo + j), tag, tm.sh, tm.err));
+			}
+			else
+				x[t] = *(in ? vl + j : vg + (lo + j));
+			c[t] = t == K ? D[l] : t < K ? lower(e, j) : U[e][l];
+		}
+		if constexpr (PKT) {
+			if (in_lo)
+				xl = vl[jl];
+			else
+				xl = res_unpack<V>(wl.y == tag ? wl.x : res_await(pk + (lo + jl), tag, tm.sh, tm.err));
+			if (in_hi)
+				xh = vl[jh];
+			else
+				xh = res_unpack<V>(wh.y == tag ? wh.x : res_await(pk + (lo + jh), tag, tm.sh, tm.err));
 		}
 		V s = V(0);
+		s = has_lo ? fma(c[0], xl, s) : s;
 #pragma unroll
-		for (int t = 0; t < K; ++t)
+		for (int t = 1; t < K; ++t)
 			s = (m >> (2 - (K - 1 - t)) & 1) ? fma(c[t], x[t], s) : s;
 		s = fma(c[K], x[K], s);
 #pragma unroll
-		for (int t = 0; t < K; ++t)
-			s = (m >> (3 + t) & 1) ? fma(c[K + 1 + t], x[K + 1 + t], s) : s;
+		for (int t = K + 1; t < 2 * K; ++t)
+			s = (m >> (3 + t - K - 1) & 1) ? fma(c[t], x[t], s) : s;
+		s = has_hi ? fma(c[2 * K], xh, s) : s;
 		return s;
 	}
 };
@@ -637,12 +650,13 @@ struct ResShape {
 	int grid, threads, rows, smem;
 };
 
-// One CTA per SM, at least kMinRows rows each (a CTA's share of a grid_sum
-// costs the same however few rows it holds); a thread per row up to
+// One CTA per SM, at least kMinRows rows each (us an iteration of CG at 32^2,
+// BiCGSTAB at 16^3 and GMRES at 48^2 with 64 / 128 / 256 / 512 rows: 6.7 / 6.4
+// / 6.7 / 7.7, 12.5 / 12.5 / 12.9 / 15.4, 13.5 / 13.5 / 13.1 / 19.6); a thread per row up to
 // kResThreads, four warps at least (one per value of a grid_sum); `per_row`
 // bytes of shared memory a row, as far as they go.
 inline ResShape res_shape(Ctx *ctx, int64_t n, int per_row, int smem_max) {
-	constexpr int kMinRows = 64;
+	constexpr int kMinRows = 128;
 	const int64_t cap = std::min(ctx->sms, kResMaxG);
 	int64_t g = std::max<int64_t>(1, std::min(cap, (n + kMinRows - 1) / kMinRows));
 	int64_t rows = ((n + g - 1) / g + 31) / 32 * 32;

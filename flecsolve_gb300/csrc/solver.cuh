@@ -121,6 +121,7 @@ struct Solver {
 	// messages and row packets of the resident kernels (on first use)
 	ResSlots *res_slots = nullptr;
 	ulonglong2 *res_pk = nullptr;
+	void *res_vals = nullptr;
 	// captured graphs, keyed by the operator they were captured with and the
 	// vectors / body they run; at most kMaxGraphs are kept (least recently
 	// launched evicted first)
@@ -162,6 +163,9 @@ int ensure_dinv(Csr *A);
 // a whole solve in one cooperative launch (resident.cu); *taken = 0: not a
 // solve for it, nothing was done
 int cg_apply_resident(Solver *s, Vec *b, Vec *x, fs_solve_info *info, int *taken);
+// the state is read back (s->hst); m: columns of a cycle (resident_gmres.cu)
+template<class T>
+int gmres_apply_resident(Solver *s, Vec *b, Vec *x, int m, bool mixed, int *taken);
 
 // host-stepped loops for operators and preconditioners the fused device
 // loops do not take (generic.cu)

@@ -133,3 +133,60 @@ def test_transpose_solve_of_a_symmetric_matrix_is_the_forward_solve(ctx, n):
     slv.apply_transpose(vb, vt)
     r = vb.numpy() - P.CSR(A.nrows, A.ncols, A.rowptr, A.col, v).to_scipy().T @ vt.numpy()
     assert np.linalg.norm(r) <= 1e-8 * np.linalg.norm(vb.numpy())
+
+
+# ------------------------------------------------------------- GMRES -----
+
+GM_SHAPES = [((5, 1, 1), 1, 0.0), ((64, 1, 1), 1, 0.0), ((12, 11, 1), 2, 0.3), ((100, 97, 1), 2, 0.0),
+             ((152, 64, 1), 2, 0.3), ((36, 41, 29), 3, 0.3), ((48, 48, 47), 3, 0.0), ((64, 64, 61), 3, 0.3),
+             ((96, 96, 95), 3, 0.3)]
+
+
+@pytest.mark.parametrize("side", ["right", "left"])
+@pytest.mark.parametrize("shape,dims,asym", GM_SHAPES)
+@pytest.mark.parametrize("method", ["gmres", "mixed_gmres"])
+def test_resident_gmres_matches_the_staged_passes(ctx, method, shape, dims, asym, side):
+    """Delayed CGS2 in one launch against the same recurrence in kernels (row
+    patterns).  FP64: counts within 2 and the estimates of the first 20 steps
+    equal to 1e-9 (rounding only); FP32 basis: the suite's bar of mixed GMRES
+    (1.2x + 30).  Either way the reported residual is the true one."""
+    A = _grid(*shape, dims, seed=sum(shape), asym=asym)
+    b = P.uniform(3, A.nrows)
+    kw = dict(maxiter=600, rtol=1e-8, max_krylov_dim=30, restart=True, ortho="dcgs2", pre_side=side)
+    one, x1, h1, l1 = _solve(ctx, A, b, method, "grid", **kw)
+    ref, x2, h2, l2 = _solve(ctx, A, b, method, "patterns", **kw)
+    assert one.status == ref.status
+    if shape[0] % 4 == 0 and A.nrows <= 450000:  # the FP32 basis's limit
+        assert l1 < l2
+    if method == "gmres":
+        assert abs(one.iters - ref.iters) <= 2
+        assert np.allclose(h1[:20], h2[:20], rtol=1e-9, atol=1e-13 * h2[0])
+    else:
+        assert one.iters <= 1.2 * ref.iters + 30
+    if one.success() and side == "right":
+        M = A.to_scipy()
+        for x in (x1, x2):
+            assert np.linalg.norm(b - M @ x) <= 1.01e-8 * np.linalg.norm(b)
+    assert one.res_norm_initial == pytest.approx(ref.res_norm_initial, rel=1e-5)
+    assert one.sol_norm_final == pytest.approx(np.linalg.norm(x1), rel=1e-5)
+
+
+@pytest.mark.parametrize("method", ["gmres", "mixed_gmres"])
+def test_resident_gmres_stops(ctx, method):
+    """Few iterations, a cycle longer than maxiter, no restart, a warm start,
+    a right-hand side of zeros: the staged passes' answers."""
+    A = _grid(48, 44, 1, 2, seed=2, asym=0.2)
+    b, x0 = P.uniform(3, A.nrows), P.uniform(4, A.nrows)
+    for kw, rhs, guess in ((dict(maxiter=0), b, None), (dict(maxiter=1), b, None), (dict(maxiter=7), b, x0),
+                           (dict(maxiter=31), b, None), (dict(maxiter=60), b, x0), (dict(maxiter=40), 0 * b, None)):
+        kw = dict(kw, rtol=1e-10, max_krylov_dim=30, restart=True, ortho="dcgs2")
+        one, x1, h1, _ = _solve(ctx, A, rhs, method, "grid", x0=guess, **kw)
+        ref, x2, h2, _ = _solve(ctx, A, rhs, method, "patterns", x0=guess, **kw)
+        assert (one.status, one.iters, one.restarts) == (ref.status, ref.iters, ref.restarts)
+        assert h1.size == h2.size
+        tol = 1e-9 if method == "gmres" else 1e-3
+        assert np.linalg.norm(x1 - x2) <= tol * max(np.linalg.norm(x2), 1e-30)
+    kw = dict(maxiter=20, rtol=1e-2, max_krylov_dim=20, restart=False, ortho="dcgs2")
+    one, x1, _, _ = _solve(ctx, A, b, method, "grid", **kw)
+    ref, x2, _, _ = _solve(ctx, A, b, method, "patterns", **kw)
+    assert (one.status, one.iters) == (ref.status, ref.iters)
