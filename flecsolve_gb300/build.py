@@ -35,7 +35,7 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
               "--expt-relaxed-constexpr",
               "-I", str(INCLUDE), "-I", str(CSRC)]
 
-CU_SOURCES = ["context.cu", "spmv.cu", "krylov.cu", "resident.cu", "resident_gmres.cu", "gmres.cu", "batched.cu", "blockcg.cu",
+CU_SOURCES = ["context.cu", "spmv.cu", "krylov.cu", "resident.cu", "resident_bicgstab.cu", "resident_gmres.cu", "gmres.cu", "batched.cu", "blockcg.cu",
               "adjoint.cu", "noalloc.cu", "matrix_market.cu", "nka.cu", "fvm.cu",
               "bdf.cu", "generic.cu", "parcsr.cu"]
 

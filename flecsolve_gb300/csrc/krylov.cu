@@ -1842,33 +1842,37 @@ static int bicgstab_apply64(Solver *s, Vec *b, Vec *x, fs_solve_info *info) {
 	const bool zg = s->set.base.use_zero_guess != 0;
 	const int PK = s->dinv64() ? 1 : 0;
 	double *res = s->w64[0], *rt = s->w64[1], *p = s->w64[2], *v = s->w64[3];
-	FS_TRY(solver_hist(s, std::max(1, s->set.base.maxiter)));
-	FS_TRY(init_state(s, s->st, (double)s->set.base.rtol, s->set.base.maxiter));
-	FS_TRY(solver_norms(s, b, x, !zg, 0));
-	if (zg) {
-		k_copy<double><<<G, kThreads, 0, ctx->stream>>>(n, (const double *)b->d, res);
-		FS_TRY(check_launch(ctx, "copy"));
-		k_fill<double><<<G, kThreads, 0, ctx->stream>>>(n, (double *)x->d, 0.0);
-		FS_TRY(check_launch(ctx, "fill"));
-	}
-	else {
-		FS_TRY(launch_spmv<double, false, false>(ctx, s->A, s->A->val, (const double *)x->d, nullptr,
-		                                         EpiResidual<double>{(const double *)b->d, res}));
-	}
-	k_bi_start<double><<<G, kThreads, 0, ctx->stream>>>(n, res, rt, p, v, s->st, s->part, s->counter);
-	FS_TRY(check_launch(ctx, "bicgstab start"));
-	FS_TRY(read_state(s));
-	int user_stop = 0;
-	if (!s->hst->done) {
-		BiArgs args{b, x, k_default(s)};
-		LoopSpec L{x, {b->d, x->d, 0}, PK ? bi_body64<1> : bi_body64<0>, &args, bi_restart, &args.k,
-		           100 + PK};
-		FS_TRY(run_loop(s, L, &user_stop));
+	int taken = 0, user_stop = 0;
+	FS_TRY(bicgstab_apply_resident(s, b, x, &taken));
+	if (!taken) {
+		FS_TRY(solver_hist(s, std::max(1, s->set.base.maxiter)));
+		FS_TRY(init_state(s, s->st, (double)s->set.base.rtol, s->set.base.maxiter));
+		FS_TRY(solver_norms(s, b, x, !zg, 0));
+		if (zg) {
+			k_copy<double><<<G, kThreads, 0, ctx->stream>>>(n, (const double *)b->d, res);
+			FS_TRY(check_launch(ctx, "copy"));
+			k_fill<double><<<G, kThreads, 0, ctx->stream>>>(n, (double *)x->d, 0.0);
+			FS_TRY(check_launch(ctx, "fill"));
+		}
+		else {
+			FS_TRY(launch_spmv<double, false, false>(ctx, s->A, s->A->val, (const double *)x->d, nullptr,
+			                                         EpiResidual<double>{(const double *)b->d, res}));
+		}
+		k_bi_start<double><<<G, kThreads, 0, ctx->stream>>>(n, res, rt, p, v, s->st, s->part, s->counter);
+		FS_TRY(check_launch(ctx, "bicgstab start"));
+		FS_TRY(read_state(s));
+		if (!s->hst->done) {
+			BiArgs args{b, x, k_default(s)};
+			LoopSpec L{x, {b->d, x->d, 0}, PK ? bi_body64<1> : bi_body64<0>, &args, bi_restart, &args.k,
+			           100 + PK};
+			FS_TRY(run_loop(s, L, &user_stop));
+		}
 	}
 	KState &h = *s->hst;
 	s->hhist_count = std::min<int64_t>((int64_t)h.nhist, s->hist_cap);
-	double xn = 0;
-	FS_TRY(sol_norm(s, x, &xn));
+	double xn = h.aux[2];
+	if (!taken)
+		FS_TRY(sol_norm(s, x, &xn));
 	memset(info, 0, sizeof(*info));
 	info->rhs_norm = (float)h.rhs_norm;
 	info->sol_norm_initial = zg ? 0.f : (float)h.sol0;

@@ -163,6 +163,8 @@ int ensure_dinv(Csr *A);
 // a whole solve in one cooperative launch (resident.cu); *taken = 0: not a
 // solve for it, nothing was done
 int cg_apply_resident(Solver *s, Vec *b, Vec *x, fs_solve_info *info, int *taken);
+// the state is read back (s->hst) (resident_bicgstab.cu)
+int bicgstab_apply_resident(Solver *s, Vec *b, Vec *x, int *taken);
 // the state is read back (s->hst); m: columns of a cycle (resident_gmres.cu)
 template<class T>
 int gmres_apply_resident(Solver *s, Vec *b, Vec *x, int m, bool mixed, int *taken);

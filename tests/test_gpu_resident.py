@@ -190,3 +190,46 @@ def test_resident_gmres_stops(ctx, method):
     one, x1, _, _ = _solve(ctx, A, b, method, "grid", **kw)
     ref, x2, _, _ = _solve(ctx, A, b, method, "patterns", **kw)
     assert (one.status, one.iters) == (ref.status, ref.iters)
+
+
+# ---------------------------------------------------------- BiCGSTAB -----
+
+@pytest.mark.parametrize("jacobi", [True, False])
+@pytest.mark.parametrize("shape,dims,asym", GM_SHAPES)
+def test_resident_bicgstab_matches_the_phase_kernels(ctx, shape, dims, asym, jacobi):
+    """The same recurrence: norms equal to 1e-9 over the first 4 iterations
+    (BiCGSTAB amplifies the rounding of its dots from there on), the stopping
+    test met by the true residual, counts within a quarter of each other."""
+    A = _grid(*shape, dims, seed=sum(shape), asym=asym)
+    b, x0 = P.uniform(3, A.nrows), P.uniform(6, A.nrows)
+    for guess in (None, x0):
+        kw = dict(maxiter=600, rtol=1e-8, x0=guess, jacobi=jacobi)
+        one, x1, h1, l1 = _solve(ctx, A, b, "bicgstab", "grid", **kw)
+        ref, x2, h2, l2 = _solve(ctx, A, b, "bicgstab", "patterns", **kw)
+        if shape[0] % 4 == 0:
+            assert l1 < l2
+        m = min(4, h1.size, h2.size)
+        assert np.allclose(h1[:m], h2[:m], rtol=1e-9, atol=1e-12 * h2[0])
+        assert one.res_norm_initial == pytest.approx(ref.res_norm_initial, rel=1e-6)
+        if one.success() and ref.success():
+            M = A.to_scipy()
+            bn = np.linalg.norm(b)
+            for x in (x1, x2):
+                assert np.linalg.norm(b - M @ x) <= 2e-8 * bn
+            assert abs(one.iters - ref.iters) <= 2 + 0.25 * ref.iters
+        assert one.sol_norm_final == pytest.approx(np.linalg.norm(x1), rel=1e-5)
+
+
+def test_resident_bicgstab_stops(ctx):
+    """No iteration, few, zeros, the unscaled early exit at a loose rtol, a
+    breakdown (r~'A P r = 0): the phase kernels' answers."""
+    A = _grid(48, 44, 1, 2, seed=2, asym=0.2)
+    b, x0 = P.uniform(3, A.nrows), P.uniform(4, A.nrows)
+    for kw, rhs, guess in ((dict(maxiter=0, rtol=1e-9), b, None), (dict(maxiter=3, rtol=1e-9), b, x0),
+                           (dict(maxiter=20, rtol=1e-9), 0 * b, None), (dict(maxiter=50, rtol=0.5), b, None),
+                           (dict(maxiter=50, rtol=0.9), 1e-3 * b, None)):
+        one, x1, h1, _ = _solve(ctx, A, rhs, "bicgstab", "grid", x0=guess, **kw)
+        ref, x2, h2, _ = _solve(ctx, A, rhs, "bicgstab", "patterns", x0=guess, **kw)
+        assert (one.status, one.iters) == (ref.status, ref.iters)
+        assert h1.size == h2.size
+        assert np.linalg.norm(x1 - x2) <= 1e-9 * max(np.linalg.norm(x2), 1e-30)
