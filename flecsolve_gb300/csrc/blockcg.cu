@@ -389,7 +389,10 @@ __device__ __forceinline__ void bcg_row4(const BcgOp<V> &A, const V *__restrict_
 		const int i = r % A.nx;
 		const int line = r / A.nx;
 		const int jj = A.K >= 2 ? line % A.ny : 0, kk = A.K >= 2 ? line / A.ny : 0;
-		const V *U1 = A.S + A.ld, *U2 = A.S + 2 * A.ld, *U3 = A.S + 3 * A.ld;
+		// the storage holds K upper diagonals: an absent dimension's (unused)
+		// coefficient is read from the diagonal, inside the allocation
+		const V *U1 = A.S + A.ld, *U2 = A.K >= 2 ? A.S + 2 * A.ld : A.S,
+		        *U3 = A.K >= 3 ? A.S + 3 * A.ld : A.S;
 		const bool has[7] = {A.K >= 3 && kk > 0, A.K >= 2 && jj > 0, i > 0, true,
 		                     i < A.nx - 1, A.K >= 2 && jj < A.ny - 1, A.K >= 3 && kk < A.nz - 1};
 		const int64_t off[7] = {-nxy, -A.nx, -1, 0, 1, A.nx, nxy};
