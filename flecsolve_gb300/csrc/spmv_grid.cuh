@@ -73,9 +73,10 @@ spmv_grid_kernel(CsrGrid<V> A, G g_in, Epi epi) {
 	const V *__restrict__ L3 = A.S + (int64_t)(A.K + 3) * A.ld;
 	for (int k = 0;; ++k) {
 		const int chunk = (int)blockIdx.x + (k / A.chunk) * (int)gridDim.x;
-		const int step = chunk * A.chunk + k % A.chunk;
-		if (step >= nstep)
+		const int at = chunk * A.chunk + k % A.chunk;
+		if (at >= nstep)
 			break;
+		const int step = epi_backwards(epi, 0) ? nstep - 1 - at : at;
 		const int s = step * kGridThreads + (int)threadIdx.x;
 		if (s >= nseg)
 			continue;

@@ -377,6 +377,17 @@ spmv_rb_kernel(CsrDev<V> A, const V *__restrict__ x, const V *__restrict__ dscal
 	}
 }
 
+// whether the grid kernel walks the rows from the last to the first (an
+// epilogue's member `backwards`; the others walk forwards)
+template<class E>
+__device__ __forceinline__ auto epi_backwards(const E &e, int) -> decltype(e.backwards) {
+	return e.backwards;
+}
+template<class E>
+__device__ __forceinline__ bool epi_backwards(const E &, long) {
+	return false;
+}
+
 // plain y = A x
 template<class V>
 struct EpiStore {
