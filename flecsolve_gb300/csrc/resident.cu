@@ -324,11 +324,9 @@ int cg_apply_resident(Solver *s, Vec *b, Vec *x, fs_solve_info *info, int *taken
 	// packets while the slice's p, r, w and x fit
 	const bool pkt = (int64_t)sh.rows * (1 + 8 * kResPktArrays) <= smem_max;
 	const Kern kern = kerns[gen][pkt][K - 1];
-	if (pkt) {
-		FS_TRY(ensure_res_packets(s));
-		a.pk = s->res_pk;
-	}
-	FS_TRY(ensure_res_slots(s));
+	if (!res_memory(s, pkt))
+		return FS_OK;
+	a.pk = pkt ? s->res_pk : nullptr;
 	FS_TRY(solver_hist(s, std::max(1, s->set.base.maxiter)));
 	a.dinv = s->dinv64();
 	a.b = (const double *)b->d;
@@ -346,8 +344,9 @@ int cg_apply_resident(Solver *s, Vec *b, Vec *x, fs_solve_info *info, int *taken
 	a.zero_guess = s->set.base.use_zero_guess != 0;
 	a.rows = sh.rows;
 	a.smem = sh.smem;
-	*taken = 1;
-	FS_TRY(res_launch(ctx, kern, sh, a, "resident cg"));
+	FS_TRY(res_launch(ctx, kern, sh, a, "resident cg", taken));
+	if (!*taken)
+		return FS_OK;
 	FS_TRY(read_state(s));
 	const KState &h = *s->hst;
 	s->hhist_count = std::min<int64_t>(h.iter, s->hist_cap);
@@ -366,29 +365,27 @@ int cg_apply_resident(Solver *s, Vec *b, Vec *x, fs_solve_info *info, int *taken
 	return FS_OK;
 }
 
-int ensure_res_slots(Solver *s) {
-	if (s->res_slots)
-		return FS_OK;
-	void *p = nullptr;
-	FS_CUDA_TRY(s->ctx, cudaMalloc(&p, sizeof(ResSlots)));
-	s->bufs.push_back(p);
-	// no slot or packet carries the epoch a first launch starts from
-	FS_CUDA_TRY(s->ctx, cudaMemsetAsync(p, 0, sizeof(ResSlots), s->ctx->stream));
-	FS_CUDA_TRY(s->ctx, cudaMemsetAsync(&((ResSlots *)p)->epoch, 1, 1, s->ctx->stream));
-	s->res_slots = (ResSlots *)p;
-	return FS_OK;
-}
-
-int ensure_res_packets(Solver *s) {
-	if (s->res_pk)
-		return FS_OK;
-	void *p = nullptr;
-	const size_t bytes = (size_t)s->n * sizeof(ulonglong2);
-	FS_CUDA_TRY(s->ctx, cudaMalloc(&p, bytes));
-	s->bufs.push_back(p);
-	FS_CUDA_TRY(s->ctx, cudaMemsetAsync(p, 0, bytes, s->ctx->stream));
-	s->res_pk = (ulonglong2 *)p;
-	return FS_OK;
+bool res_memory(Solver *s, bool packets) {
+	// one buffer of zeroes; false (and no error left) when there is no room
+	auto get = [&](size_t bytes) -> void * {
+		void *p = nullptr;
+		if (cudaMalloc(&p, bytes) != cudaSuccess) {
+			cudaGetLastError();
+			return nullptr;
+		}
+		s->bufs.push_back(p);
+		return cudaMemsetAsync(p, 0, bytes, s->ctx->stream) == cudaSuccess ? p : nullptr;
+	};
+	if (!s->res_slots) {
+		// no slot or packet carries the epoch a first launch starts from
+		auto *p = (ResSlots *)get(sizeof(ResSlots));
+		if (!p || cudaMemsetAsync(&p->epoch, 1, 1, s->ctx->stream) != cudaSuccess)
+			return false;
+		s->res_slots = p;
+	}
+	if (packets && !s->res_pk)
+		s->res_pk = (ulonglong2 *)get((size_t)s->n * sizeof(ulonglong2));
+	return !packets || s->res_pk;
 }
 
 }  // namespace fsg

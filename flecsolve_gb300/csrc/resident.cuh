@@ -670,8 +670,11 @@ inline ResShape res_shape(Ctx *ctx, int64_t n, int per_row, int smem_max) {
 	return s;
 }
 
+// `taken` = 0: the device has no room for every CTA at once (SMs set aside for
+// another client), and the caller's phase kernels run instead
 template<class Args>
-inline int res_launch(Ctx *ctx, void (*kern)(Args), const ResShape &sh, const Args &a, const char *what) {
+inline int res_launch(Ctx *ctx, void (*kern)(Args), const ResShape &sh, const Args &a, const char *what,
+                      int *taken) {
 	cudaLaunchConfig_t cfg{};
 	cfg.gridDim = dim3((unsigned)sh.grid);
 	cfg.blockDim = dim3((unsigned)sh.threads);
@@ -682,7 +685,13 @@ inline int res_launch(Ctx *ctx, void (*kern)(Args), const ResShape &sh, const Ar
 	at[0].val.cooperative = 1;
 	cfg.attrs = at;
 	cfg.numAttrs = 1;
-	return check_launch_rc(ctx, cudaLaunchKernelEx(&cfg, kern, a), what);
+	const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a);
+	*taken = e != cudaErrorCooperativeLaunchTooLarge;
+	if (!*taken) {
+		cudaGetLastError();
+		return FS_OK;
+	}
+	return check_launch_rc(ctx, e, what);
 }
 
 // dynamic shared memory a resident kernel may use (its static part is taken
@@ -738,8 +747,9 @@ inline bool res_grid(const Csr *A, ResGrid<V> &g, bool &gen) {
 	return true;
 }
 
-// the solver's messages and row packets, allocated on first use (resident.cu)
-int ensure_res_slots(Solver *s);
-int ensure_res_packets(Solver *s);
+// the solver's messages (and row packets), allocated on first use
+// (resident.cu); false when there is no memory for them: the caller's phase
+// kernels, which need neither, run instead
+bool res_memory(Solver *s, bool packets);
 
 }  // namespace fsg

@@ -420,8 +420,8 @@ int bicgstab_apply_resident(Solver *s, Vec *b, Vec *x, int *taken) {
 	const ResShape sh = res_shape(ctx, s->n, per_row, smem_max);
 	if ((int64_t)sh.rows * (1 + 16) > smem_max)
 		return FS_OK;
-	FS_TRY(ensure_res_slots(s));
-	FS_TRY(ensure_res_packets(s));
+	if (!res_memory(s, true))
+		return FS_OK;
 	FS_TRY(solver_hist(s, std::max(1, s->set.base.maxiter)));
 	a.dinv = s->dinv64();
 	a.b = (const double *)b->d;
@@ -442,8 +442,9 @@ int bicgstab_apply_resident(Solver *s, Vec *b, Vec *x, int *taken) {
 	a.zero_guess = s->set.base.use_zero_guess != 0;
 	a.rows = sh.rows;
 	a.smem = sh.smem;
-	*taken = 1;
-	FS_TRY(res_launch(ctx, kern, sh, a, "resident bicgstab"));
+	FS_TRY(res_launch(ctx, kern, sh, a, "resident bicgstab", taken));
+	if (!*taken)
+		return FS_OK;
 	return read_state(s);
 }
 

@@ -731,11 +731,14 @@ int gmres_apply_resident(Solver *s, Vec *b, Vec *x, int m, bool mixed, int *take
 	if ((int64_t)sh.rows * (1 + 2 * (int)sizeof(T)) > smem_max)
 		return FS_OK;
 	sh.threads = kRgThreads;
-	FS_TRY(ensure_res_slots(s));
-	FS_TRY(ensure_res_packets(s));
+	if (!res_memory(s, true))
+		return FS_OK;
 	if (!s->res_vals) {
 		void *p = nullptr;
-		FS_CUDA_TRY(ctx, cudaMalloc(&p, sizeof(RgSlots)));
+		if (cudaMalloc(&p, sizeof(RgSlots)) != cudaSuccess) {
+			cudaGetLastError();
+			return FS_OK;  // no room: the phase kernels
+		}
 		s->bufs.push_back(p);
 		FS_CUDA_TRY(ctx, cudaMemsetAsync(p, 0, sizeof(RgSlots), ctx->stream));
 		s->res_vals = p;
@@ -766,8 +769,9 @@ int gmres_apply_resident(Solver *s, Vec *b, Vec *x, int m, bool mixed, int *take
 	a.mixed = mixed;
 	a.rows = sh.rows;
 	a.smem = sh.smem;
-	*taken = 1;
-	FS_TRY(res_launch(ctx, kern, sh, a, "resident gmres"));
+	FS_TRY(res_launch(ctx, kern, sh, a, "resident gmres", taken));
+	if (!*taken)
+		return FS_OK;
 	return read_state(s);
 }
 
