@@ -1,5 +1,10 @@
-// Batched solves: many independent systems of uneven size in one persistent
-// launch.
+// Batched solves: many independent systems of uneven size, each solved by a
+// cluster or a CTA that stays with it.
+//
+// A batch whose systems are all symmetric 5-point stencils on square grids of up
+// to 180,000 rows is solved on chip (batched_grid.cuh), one launch for each
+// cluster size.  What follows describes the kernel for every other batch and
+// for schedules given by the caller, one persistent launch.
 //
 // The systems are the diagonal blocks of one block-diagonal CSR matrix
 // (rows [off[s], off[s+1]) couple only among themselves).  A team owns one
@@ -55,6 +60,7 @@ struct BatchArgs {
 	int nsys;
 	int nbig;                // systems 0..nbig-1 of `order` own a whole cluster
 	const int *order;        // system processed by cluster c (largest first)
+	int first;               // grid kernel: cluster c takes order[first + c]
 	const int64_t *off;      // row offsets, nsys + 1
 	const int *rowptr;
 	const int *col;
@@ -80,6 +86,16 @@ struct BatchArgs {
 	const double *gd64, *gu1_64, *gu2_64;
 	const float *gd32, *gu1_32, *gu2_32;
 };
+
+}  // namespace
+
+}  // namespace fsg
+
+#include "batched_grid.cuh"
+
+namespace fsg {
+
+namespace {
 
 __device__ __forceinline__ float fmav(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fmav(double a, double b, double c) { return fma(a, b, c); }
@@ -554,6 +570,7 @@ struct BatchPlan {
 	int nsys = 0;
 	int tuned_cluster = 0, tuned_threads = 0;
 	int tuned_nbig = -1;  // systems that own a whole cluster (-1: all)
+	bool ruled = false;   // the three stand for `classes`, not for a tuning
 	// grid-stencil storage (every system a 5-point s x s grid with symmetric
 	// values): per-system sides, diagonal and upper diagonals; `grid` is 1
 	// when it holds for the values of generation `grid_gen`, 0 when not, -1
@@ -564,9 +581,23 @@ struct BatchPlan {
 	unsigned *d_bad = nullptr;
 	int grid = -1;
 	unsigned grid_gen = 0;
+	// the grid kernel's launches: systems order[first, first + count) on
+	// `team` CTAs each, each launch on a stream of its own (empty: not for it)
+	struct Class {
+		int first, count, team;
+		int64_t smem;
+	};
+	std::vector<Class> classes;
+	bool classed = false;
+	std::vector<cudaStream_t> streams;
+	std::vector<cudaEvent_t> events;
 };
 
 void free_plan(BatchPlan &p) {
+	for (cudaStream_t q : p.streams)
+		cudaStreamDestroy(q);
+	for (cudaEvent_t e : p.events)
+		cudaEventDestroy(e);
 	for (void *q : {(void *)p.d_off, (void *)p.d_order, (void *)p.d_info, (void *)p.work,
 	                (void *)p.work64, (void *)p.d_side, (void *)p.g64, (void *)p.g32, (void *)p.d_bad})
 		if (q)
@@ -641,6 +672,122 @@ int launch_batch(Ctx *ctx, const BatchArgs &a, int nsys, int cluster, int thread
 		               threads, cudaGetErrorString(e));
 	ctx->launches++;
 	return FS_OK;
+}
+
+cudaLaunchConfig_t grid_config(const BatchPlan::Class &c, cudaStream_t stream, cudaLaunchAttribute *at) {
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3((unsigned)(c.count * c.team), 1, 1);
+	cfg.blockDim = dim3((unsigned)kBgThreads, 1, 1);
+	cfg.dynamicSmemBytes = (size_t)c.smem;
+	cfg.stream = stream;
+	at[0].id = cudaLaunchAttributeClusterDimension;
+	at[0].val.clusterDim.x = (unsigned)c.team;
+	at[0].val.clusterDim.y = 1;
+	at[0].val.clusterDim.z = 1;
+	cfg.attrs = at;
+	cfg.numAttrs = 1;
+	return cfg;
+}
+
+// The grid kernel's launches of a plan on grid storage: the systems in order of
+// size, cut where the team changes; none (the kernel above, autotuned) when one
+// of them is too large or the device cannot run a cluster.  A slice takes as
+// many rows as a CTA holds when the batch fills the GPU, and what gives every
+// SM some of them when it does not, 1,024 at least: 32 systems of side 32..64
+// take 3.0, 2.3, 2.2, 2.3 and 2.5 ms with 4,096, 2,048, 1,024, 512 and 256, and
+// 32 of side 32..256 take 15.4 ms with clusters of up to 16 CTAs, 21.9 ms with
+// up to 8.  The general kernel's best schedules: 4.2 and 47.7 ms.  CTAs of 256
+// and 128 threads, two and four an SM, for the small systems of a large batch
+// change nothing at 512 systems of side 32..256 (144.6 and 143.8 ms) and lose
+// at 400 of side 32..64 (6.4 and 5.1 ms).
+constexpr int64_t kBgMinRows = 1024;
+
+void plan_classes(Ctx *ctx, BatchPlan &p, const std::vector<int> &order) {
+	p.classes.clear();
+	p.classed = true;
+	const int64_t cap = (int64_t)kBgRows * kBgThreads;
+	const int64_t want = std::min(cap, std::max(kBgMinRows, p.off[p.nsys] / ctx->sms));
+	std::vector<BatchPlan::Class> cls;
+	const int64_t room = res_smem_max(ctx, k_batch_grid);
+	// clusters of more than 8 CTAs are an opt-in
+	const int most = cudaFuncSetAttribute(k_batch_grid, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+	                         cudaSuccess
+	                     ? kBgTeam : 8;
+	cudaGetLastError();
+	for (int k = 0; k < p.nsys; ++k) {
+		const int64_t n = p.off[order[k] + 1] - p.off[order[k]];
+		const int64_t s = (int64_t)std::llround(std::sqrt((double)n));
+		BatchPlan::Class c{k, 1, 1, 0};
+		c.team = (int)std::min<int64_t>(most, std::max<int64_t>(1, (n + want - 1) / want));
+		while (c.team > 1 && bg_rows(n, c.team) < s)
+			--c.team;
+		auto fits = [&]() {
+			c.smem = bg_smem(bg_rows(n, c.team), s);
+			return bg_rows(n, c.team) <= cap && c.smem <= room;
+		};
+		while (!fits() && c.team < most)
+			++c.team;
+		if (!fits())
+			return;
+		if (!cls.empty() && cls.back().team == c.team) {
+			cls.back().count++;
+			cls.back().smem = std::max(cls.back().smem, c.smem);
+		}
+		else
+			cls.push_back(c);
+	}
+	for (const auto &c : cls) {
+		cudaLaunchAttribute at[1];
+		const cudaLaunchConfig_t cfg = grid_config(c, ctx->stream, at);
+		int active = 0;
+		if (cudaOccupancyMaxActiveClusters(&active, k_batch_grid, &cfg) != cudaSuccess || active < 1) {
+			cudaGetLastError();
+			return;
+		}
+	}
+	// a stream for each launch after the first, an event to start and one to
+	// end each
+	while (p.streams.size() + 1 < cls.size()) {
+		cudaStream_t q;
+		if (cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) != cudaSuccess) {
+			cudaGetLastError();
+			return;
+		}
+		p.streams.push_back(q);
+	}
+	while (p.events.size() < cls.size()) {
+		cudaEvent_t e;
+		if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+			cudaGetLastError();
+			return;
+		}
+		p.events.push_back(e);
+	}
+	p.classes = cls;
+}
+
+// The launches side by side, the largest systems first; ctx->stream goes on
+// when all are done, also when one could not be launched.
+int launch_classes(Ctx *ctx, const BatchArgs &a, const BatchPlan &p) {
+	FS_CUDA_TRY(ctx, cudaEventRecord(p.events[0], ctx->stream));
+	cudaError_t e = cudaSuccess;
+	size_t k = 0;
+	for (; k < p.classes.size() && e == cudaSuccess; ++k) {
+		cudaStream_t q = k ? p.streams[k - 1] : ctx->stream;
+		if (k && (e = cudaStreamWaitEvent(q, p.events[0], 0)) != cudaSuccess)
+			break;
+		cudaLaunchAttribute at[1];
+		const cudaLaunchConfig_t cfg = grid_config(p.classes[k], q, at);
+		BatchArgs b = a;
+		b.first = p.classes[k].first;
+		e = cudaLaunchKernelEx(&cfg, k_batch_grid, b);
+		ctx->launches += e == cudaSuccess;
+	}
+	for (size_t i = 1; i < k; ++i) {
+		FS_CUDA_TRY(ctx, cudaEventRecord(p.events[i], p.streams[i - 1]));
+		FS_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, p.events[i], 0));
+	}
+	return e == cudaSuccess ? FS_OK : check_launch_rc(ctx, e, "batched CG on grids");
 }
 
 // cluster_systems: -1 chooses (with the sizes), else that many of the
@@ -731,6 +878,7 @@ int batch_solve(fs_ctx h, const fs_krylov_settings *s, fs_csr Ah, int nsys, cons
 	a.delta = s->inner_rtol > 0 ? s->inner_rtol : 0.1;
 	a.zero_guess = s->base.use_zero_guess ? 1 : 0;
 	a.nbig = cluster_systems >= 0 ? cluster_systems : nsys;
+	a.first = 0;
 	a.side = nullptr;
 	a.gd64 = a.gu1_64 = a.gu2_64 = nullptr;
 	a.gd32 = a.gu1_32 = a.gu2_32 = nullptr;
@@ -746,8 +894,34 @@ int batch_solve(fs_ctx h, const fs_krylov_settings *s, fs_csr Ah, int nsys, cons
 	}
 
 	int cl = cluster_size, th = threads;
+	if (!cl && !th && cluster_systems < 0 && p.grid == 1) {
+		if (!p.classed) {
+			std::vector<int> order(nsys);
+			FS_CUDA_TRY(ctx, cudaMemcpy(order.data(), p.d_order, sizeof(int) * nsys, cudaMemcpyDeviceToHost));
+			plan_classes(ctx, p, order);
+		}
+		if (!p.classes.empty()) {
+			// for fs_batch_schedule: the closest schedule with given sizes
+			p.ruled = true;
+			p.tuned_threads = kBgThreads;
+			p.tuned_cluster = 1;
+			while (p.tuned_cluster < std::min(8, p.classes[0].team))
+				p.tuned_cluster *= 2;
+			p.tuned_nbig = 1;
+			for (const auto &c : p.classes)
+				if (c.team > 1)
+					p.tuned_nbig = c.first + c.count;
+			FS_TRY(launch_classes(ctx, a, p));
+			FS_CUDA_TRY(ctx, cudaMemcpyAsync(infos, p.d_info, sizeof(fs_solve_info) * nsys,
+			                                 cudaMemcpyDeviceToHost, ctx->stream));
+			FS_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+			return FS_OK;
+		}
+	}
 	if (cl == 0 || th == 0) {
-		if (p.tuned_cluster == 0) {
+		if (p.tuned_cluster == 0 || p.ruled) {
+			p.tuned_cluster = 0;
+			p.ruled = false;
 			// autotuner, stage 1: time a short capped run of each cluster /
 			// CTA size (every system a whole cluster) on this batch and keep
 			// the fastest cluster size for each CTA size; the solution is

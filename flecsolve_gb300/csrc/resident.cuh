@@ -142,8 +142,21 @@ __device__ __forceinline__ ResFix res_fix_cta(ResFix f) {
 	return {hi * (1 << 13) + ((lo + (1ll << 32)) >> 33), E};
 }
 
-// (hi 2^16 + lo 2^-30) 2^(E - 1075)
+// (hi 2^16 + lo 2^-30) 2^(E - 1075), rounded to nearest (0 <= lo < 2^46).  In
+// integers: the conversions, the product and the sum of the FP64 form below
+// it take 62 cycles each.
 __device__ __forceinline__ double res_fix_double(long long hi, long long lo, int E) {
+	const bool neg = hi < 0;
+	const unsigned long long l = (unsigned long long)(neg ? -lo & ((1ll << 46) - 1) : lo) << 18;
+	const unsigned long long h = (unsigned long long)(neg ? -hi - (lo != 0) : hi);
+	const int z = __clzll((long long)h), ex = E - z + 27;
+	if (h != 0 && ex > 0 && ex < 0x7fe) {
+		const unsigned long long m = z ? h << z | l >> (64 - z) : h, rest = l << z;
+		const unsigned r = (unsigned)m & 0x7ff;
+		const unsigned long long up = r > 0x400 || (r == 0x400 && ((m & 0x800) || rest));
+		return __longlong_as_double((long long)((m >> 11) + ((unsigned long long)(ex - 1) << 52) + up |
+		                                        (unsigned long long)neg << 63));
+	}
 	const double t = fma((double)lo, 0x1p-46, (double)hi);
 	const int k = E - 1059;
 	if (k >= -1022)
@@ -248,24 +261,37 @@ __device__ __forceinline__ double res_fix_grid(const ResFix (&f)[Q]) {
 	return res_fix_double(hi, lo, E - F);
 }
 
-// the sum of 8 floats a lane over a warp, F = 3 (29 bits below the unit of
+// a sum's value, F = 0
+__device__ __forceinline__ double res_fix_value(ResFix f) {
+	if (f.e == 0x7ff) {
+		const double inf = __longlong_as_double(0x7ff0000000000000ll);
+		return (f.q & 4) || (f.q & 3) == 3 ? __longlong_as_double(0x7ff8000000000000ll)
+		                                   : (f.q & 1) ? inf : -inf;
+	}
+	// q = hi 2^16 + lo 2^-30
+	return res_fix_double(f.q >> 16, (f.q & 0xffff) << 30, f.e);
+}
+
+// the sum of N <= 8 floats a lane over a warp, F = 3 (29 bits below the unit of
 // the largest: 24 + 29 + 8 bits, below 2^62)
-__device__ __forceinline__ ResFix res_fix_warp8(const float (&v)[8]) {
+template<int N>
+__device__ __forceinline__ ResFix res_fix_warp(const float (&v)[N]) {
+	static_assert(N <= 8, "");
 	int E = 1;
 #pragma unroll
-	for (int i = 0; i < 8; ++i)
+	for (int i = 0; i < N; ++i)
 		E = max(E, (__float_as_int(v[i]) >> 23) & 0xff);
 	E = __reduce_max_sync(0xffffffffu, E);
 	if (E == 0xff) {
 		int cls = 0;
 #pragma unroll
-		for (int i = 0; i < 8; ++i)
+		for (int i = 0; i < N; ++i)
 			cls |= isnan(v[i]) ? 4 : isinf(v[i]) ? (v[i] < 0.f ? 2 : 1) : 0;
 		return res_special(cls);
 	}
 	long long q = 0;
 #pragma unroll
-	for (int i = 0; i < 8; ++i) {
+	for (int i = 0; i < N; ++i) {
 		const int b = __float_as_int(v[i]), e = (b >> 23) & 0xff;
 		const int m = (b & 0x7fffff) | (e ? 0x800000 : 0);
 		const int d = min(E - max(e, 1), 63);

@@ -110,7 +110,7 @@ struct RgAcc<float> {
 	}
 	__device__ ResFix sum() const {
 		const float v[8] = {hi[0], hi[1], hi[2], hi[3], lo[0], lo[1], lo[2], lo[3]};
-		return res_fix_warp8(v);
+		return res_fix_warp(v);
 	}
 };
 
