@@ -279,10 +279,11 @@ __global__ void k_inner_init(KState *in, const KState *out, double inner_rtol, i
 // products, the replacement test) and k_cg_dir_x (the solution step
 // xs += alpha p and the direction update).
 
-// x64 += xs; xs = 0
-__global__ void k_rel_fold(int64_t n, double *__restrict__ x, float *__restrict__ xs) {
+// x64 += xs (or D^-1 xs); xs = 0
+__global__ void k_rel_fold(int64_t n, double *__restrict__ x, float *__restrict__ xs,
+                           const double *__restrict__ dinv) {
 	FOR_EACH(i, n) {
-		x[i] += (double)xs[i];
+		x[i] = dinv ? fma(dinv[i], (double)xs[i], x[i]) : x[i] + (double)xs[i];
 		xs[i] = 0.f;
 	}
 }
@@ -539,10 +540,12 @@ k_bi_start(int64_t n, const V *__restrict__ res, V *__restrict__ rt, V *__restri
 	}
 }
 
-// p update (bicgstab.hh:115-122)
-template<class V>
+// p update (bicgstab.hh:115-122).  BACK: rows from the last to the first.
+template<class V, bool BACK = false>
 __global__ void k_bi_p(int64_t n, V *__restrict__ p, const V *__restrict__ v,
                        const V *__restrict__ res, const KState *st) {
+	pdl_wait();
+	pdl_trigger();
 	if (stopped(st))
 		return;
 	if (st->iter == 0) {
@@ -559,7 +562,8 @@ __global__ void k_bi_p(int64_t n, V *__restrict__ p, const V *__restrict__ v,
 			float4 *p4 = reinterpret_cast<float4 *>(p);
 			const float4 *v4 = reinterpret_cast<const float4 *>(v);
 			const float4 *r4 = reinterpret_cast<const float4 *>(res);
-			FOR_EACH(i, n4) {
+			FOR_EACH(e, n4) {
+				const int64_t i = BACK ? n4 - 1 - e : e;
 				float4 pv = p4[i];
 				const float4 vv = v4[i], rv = r4[i];
 				one(pv.x, vv.x, rv.x);
@@ -587,6 +591,7 @@ struct EpiBiV {
 	KState *st;
 	double *part;
 	unsigned *counter;
+	bool backwards = false;
 	__device__ bool skip() const { return stopped(st); }
 	template<class A>
 	__device__ void row(int r, V s, A &acc) const {
@@ -605,11 +610,13 @@ struct EpiBiV {
 };
 
 // s = res - alpha v, s_norm; early exit when s_norm < rtol (bicgstab.hh:132-143)
-template<class V>
+template<class V, bool BACK = false>
 __global__ void __launch_bounds__(kThreads)
 k_bi_s(int64_t n, V *__restrict__ s, const V *__restrict__ v, const V *__restrict__ res,
        KState *st, double *part, unsigned *counter) {
 	__shared__ double sh[128];
+	pdl_wait();
+	pdl_trigger();
 	if (stopped(st))
 		return;
 	const V a = (V)st->alpha;
@@ -625,7 +632,8 @@ k_bi_s(int64_t n, V *__restrict__ s, const V *__restrict__ v, const V *__restric
 		float4 *s4 = reinterpret_cast<float4 *>(s);
 		const float4 *v4 = reinterpret_cast<const float4 *>(v);
 		const float4 *r4 = reinterpret_cast<const float4 *>(res);
-		FOR_EACH(i, n4) {
+		FOR_EACH(e, n4) {
+			const int64_t i = BACK ? n4 - 1 - e : e;
 			float4 sv;
 			const float4 vv = v4[i], rv = r4[i];
 			one(sv.x, vv.x, rv.x);
@@ -664,6 +672,7 @@ struct EpiBiT {
 	KState *st;
 	double *part;
 	unsigned *counter;
+	bool backwards = false;
 	__device__ bool skip() const { return stopped(st) || (st->flags & KF_EARLY); }
 	template<class A>
 	__device__ void row(int r, V val, A &acc) const {
@@ -686,13 +695,15 @@ struct EpiBiT {
 // raises KF_RELIABLE with the reason in aux[3] (0 drop, 1 converged, 2 early
 // exit, 3 omega == 0, 4 maxiter) and the host replaces the residual by the
 // FP64 one before deciding.
-template<class V, int PK, bool RELY = false>
+template<class V, int PK, bool RELY = false, bool BACK = false>
 __global__ void __launch_bounds__(kThreads)
 k_bi_x(int64_t n, V *__restrict__ x, const V *__restrict__ p, const V *__restrict__ s,
        const V *__restrict__ t, V *__restrict__ res, const V *__restrict__ rt,
        const V *__restrict__ dinv, KState *st, double *part, unsigned *counter,
        double *hist) {
 	__shared__ double sh[128];
+	pdl_wait();
+	pdl_trigger();
 	if (stopped(st))
 		return;
 	const V a = (V)st->alpha;
@@ -736,7 +747,8 @@ k_bi_x(int64_t n, V *__restrict__ x, const V *__restrict__ p, const V *__restric
 		const float4 *t4 = reinterpret_cast<const float4 *>(t);
 		const float4 *q4 = reinterpret_cast<const float4 *>(rt);
 		const float4 *d4 = reinterpret_cast<const float4 *>(dinv);
-		FOR_EACH(i, n4) {
+		FOR_EACH(e, n4) {
+			const int64_t i = BACK ? n4 - 1 - e : e;
 			float4 xv = x4[i], rv;
 			const float4 pv = p4[i], sv = s4[i], tv = t4[i], qv = q4[i];
 			const float4 dv = PK ? d4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1812,25 +1824,27 @@ static int bi_body64(Solver *s, void *a) {
 	const double *dinv = s->dinv64();
 	const int G = red_grid(ctx, n);
 	for (int k = 0; k < g->k; ++k) {
-		k_bi_p<double><<<G, kThreads, 0, ctx->stream>>>(n, p, v, res, s->st);
-		FS_TRY(check_launch(ctx, "bicgstab p"));
+		FS_TRY(check_launch_rc(ctx, launch_pdl(ctx->stream, k_bi_p<double>, G, kThreads, 0, n, p, v, res,
+		                                       (const KState *)s->st),
+		                       "bicgstab p"));
 		if (PK)
 			FS_TRY((launch_spmv<double, false, true>(ctx, s->A, s->A->val, p, dinv,
 			                                         EpiBiV<double>{v, rt, s->st, s->part, s->counter})));
 		else
 			FS_TRY((launch_spmv<double, false, false>(ctx, s->A, s->A->val, p, nullptr,
 			                                          EpiBiV<double>{v, rt, s->st, s->part, s->counter})));
-		k_bi_s<double><<<G, kThreads, 0, ctx->stream>>>(n, sv, v, res, s->st, s->part, s->counter);
-		FS_TRY(check_launch(ctx, "bicgstab s"));
+		FS_TRY(check_launch_rc(ctx, launch_pdl(ctx->stream, k_bi_s<double>, G, kThreads, 0, n, sv, v, res,
+		                                       s->st, s->part, s->counter),
+		                       "bicgstab s"));
 		if (PK)
 			FS_TRY((launch_spmv<double, false, true>(ctx, s->A, s->A->val, sv, dinv,
 			                                         EpiBiT<double>{t, sv, s->st, s->part, s->counter})));
 		else
 			FS_TRY((launch_spmv<double, false, false>(ctx, s->A, s->A->val, sv, nullptr,
 			                                          EpiBiT<double>{t, sv, s->st, s->part, s->counter})));
-		k_bi_x<double, PK><<<G, kThreads, 0, ctx->stream>>>(n, x, p, sv, t, res, rt, dinv, s->st,
-		                                                   s->part, s->counter, s->hist);
-		FS_TRY(check_launch(ctx, "bicgstab x"));
+		FS_TRY(check_launch_rc(ctx, launch_pdl(ctx->stream, k_bi_x<double, PK>, G, kThreads, 0, n, x, p,
+		                                       sv, t, res, rt, dinv, s->st, s->part, s->counter, s->hist),
+		                       "bicgstab x"));
 	}
 	return FS_OK;
 }
@@ -1910,6 +1924,55 @@ static int bicgstab_apply64(Solver *s, Vec *b, Vec *x, fs_solve_info *info) {
 
 // ------------------------------------------- mixed precision BiCGSTAB --
 
+// The general grid storage with column c scaled by D^-1(c): right Jacobi
+// preconditioning in the values, from the FP64 ones, rounded once.  Bound: HBM.
+// It takes the seven scale loads a row from both SpMVs of an iteration (54 and
+// 47 us at 192^3 with them, 51 and 45 without) and D^-1 from three passes: with
+// the passes launched ahead and walking against each other, 201 -> 170 us an
+// iteration, against 137 us of memory traffic.
+__global__ void k_scale_cols(int n, int K, int d2, int d3, int64_t ld, const double *__restrict__ S,
+                             const double *__restrict__ dinv, float *__restrict__ out) {
+	const int off[4] = {0, 1, d2, d3};
+	FOR_EACH(i, n) {
+		const int r = (int)i;
+		out[r] = (float)(S[r] * dinv[r]);
+		for (int k = 1; k <= K; ++k) {
+			const int64_t up = k * ld + r, lo = (K + k) * ld + r;
+			if (r + off[k] < n)
+				out[up] = (float)(S[up] * dinv[r + off[k]]);
+			if (r >= off[k])
+				out[lo] = (float)(S[lo] * dinv[r - off[k]]);
+		}
+	}
+}
+
+// Builds it for a solve (60 us at 192^3, each time: the values or D^-1 may
+// have changed); null when the operator is not in that storage or there is no
+// memory: the SpMV then scales the vector as it reads it.
+static const float *bi_scaled(Solver *s) {
+	Csr *A = s->A;
+	if (!s->dinv64() || ensure_sym(A, false) != FS_OK || !A->gen64_valid ||
+	    active_coding(A, true) != kCodingGridGen || !grid_aligned<float>(A, s->w32[2], nullptr))
+		return nullptr;
+	const size_t len = (size_t)(2 * A->nsym + 1) * (size_t)A->sym_ld;
+	if (s->scaled_len < len) {
+		void *p = nullptr;
+		if (cudaMalloc(&p, len * sizeof(float)) != cudaSuccess) {
+			cudaGetLastError();
+			return nullptr;
+		}
+		s->bufs.push_back(p);
+		s->scaled = (float *)p;
+		s->scaled_len = len;
+	}
+	k_scale_cols<<<grid_for(s->ctx, s->n, 256, 4), 256, 0, s->ctx->stream>>>(
+		(int)s->n, A->nsym, A->grid_nx, A->grid_nx * A->grid_ny, A->sym_ld, A->gen64, s->dinv64(),
+		s->scaled);
+	return check_launch(s->ctx, "scaled grid storage") == FS_OK ? s->scaled : nullptr;
+}
+
+// PK: 0 no preconditioner, 1 the SpMV scales the vector it reads, 2 the values
+// are scaled (xs then holds D times the correction)
 template<int PK>
 static int bi_body32(Solver *s, void *a) {
 	BiArgs *g = (BiArgs *)a;
@@ -1917,28 +1980,38 @@ static int bi_body32(Solver *s, void *a) {
 	const int64_t n = s->n;
 	float *res = s->w32[0], *rt = s->w32[1], *p = s->w32[2], *v = s->w32[3], *sv = s->w32[4],
 	      *t = s->w32[5], *xs = s->w32[6];
-	const float *dinv = s->dinv32();
+	const float *dinv = PK == 1 ? s->dinv32() : nullptr;
 	const int G = red_grid(ctx, n);
+	auto spmv = [&](const float *x, const auto &epi) -> int {
+		if constexpr (PK == 2)
+			return launch_spmv_grid<float, false, true>(ctx, s->A, GatherX<float>{x}, epi,
+			                                            (const float *)s->scaled);
+		else
+			return launch_spmv<float, false, PK == 1>(ctx, s->A, s->A->val32, x, dinv, epi);
+	};
+	// the passes alternate direction, as in mixed CG
+	bool back = false;
 	for (int k = 0; k < g->k; ++k) {
-		k_bi_p<float><<<G, kThreads, 0, ctx->stream>>>(n, p, v, res, s->st);
-		FS_TRY(check_launch(ctx, "bicgstab p f32"));
-		if (PK)
-			FS_TRY((launch_spmv<float, false, true>(ctx, s->A, s->A->val32, p, dinv,
-			                                        EpiBiV<float>{v, rt, s->st, s->part, s->counter})));
-		else
-			FS_TRY((launch_spmv<float, false, false>(ctx, s->A, s->A->val32, p, nullptr,
-			                                         EpiBiV<float>{v, rt, s->st, s->part, s->counter})));
-		k_bi_s<float><<<G, kThreads, 0, ctx->stream>>>(n, sv, v, res, s->st, s->part, s->counter);
-		FS_TRY(check_launch(ctx, "bicgstab s f32"));
-		if (PK)
-			FS_TRY((launch_spmv<float, false, true>(ctx, s->A, s->A->val32, sv, dinv,
-			                                        EpiBiT<float>{t, sv, s->st, s->part, s->counter})));
-		else
-			FS_TRY((launch_spmv<float, false, false>(ctx, s->A, s->A->val32, sv, nullptr,
-			                                         EpiBiT<float>{t, sv, s->st, s->part, s->counter})));
-		k_bi_x<float, PK, true><<<G, kThreads, 0, ctx->stream>>>(n, xs, p, sv, t, res, rt, dinv, s->st,
-		                                                        s->part, s->counter, s->hist);
-		FS_TRY(check_launch(ctx, "bicgstab x f32"));
+		FS_TRY(check_launch_rc(ctx, launch_pdl(ctx->stream, back ? k_bi_p<float, true> : k_bi_p<float, false>,
+		                                       G, kThreads, 0, n, p, v, res, (const KState *)s->st),
+		                       "bicgstab p f32"));
+		back = !back;
+		FS_TRY(spmv(p, EpiBiV<float>{v, rt, s->st, s->part, s->counter, back}));
+		back = !back;
+		FS_TRY(check_launch_rc(ctx, launch_pdl(ctx->stream, back ? k_bi_s<float, true> : k_bi_s<float, false>,
+		                                       G, kThreads, 0, n, sv, v, res, s->st, s->part, s->counter),
+		                       "bicgstab s f32"));
+		back = !back;
+		FS_TRY(spmv(sv, EpiBiT<float>{t, sv, s->st, s->part, s->counter, back}));
+		back = !back;
+		constexpr int PX = PK == 1;
+		FS_TRY(check_launch_rc(ctx,
+		                       launch_pdl(ctx->stream,
+		                                  back ? k_bi_x<float, PX, true, true> : k_bi_x<float, PX, true, false>,
+		                                  G, kThreads, 0, n, xs, p, sv, t, res, rt, dinv, s->st, s->part,
+		                                  s->counter, s->hist),
+		                       "bicgstab x f32"));
+		back = !back;
 	}
 	return FS_OK;
 }
@@ -1952,7 +2025,8 @@ static int bicgstab_apply_reliable(Solver *s, Vec *b, Vec *x, fs_solve_info *inf
 	const int64_t n = s->n;
 	const int G = red_grid(ctx, n);
 	const bool zg = s->set.base.use_zero_guess != 0;
-	const int PK = s->dinv32() ? 1 : 0;
+	const int PK = !s->dinv32() ? 0 : bi_scaled(s) ? 2 : 1;
+	const double *fold = PK == 2 ? s->dinv64() : nullptr;
 	float *res = s->w32[0], *rt = s->w32[1], *p = s->w32[2], *v = s->w32[3], *xs = s->w32[6];
 	const int maxiter = s->set.base.maxiter;
 	const double delta = s->set.inner_rtol > 0 ? s->set.inner_rtol : 1e-2;
@@ -1964,7 +2038,7 @@ static int bicgstab_apply_reliable(Solver *s, Vec *b, Vec *x, fs_solve_info *inf
 		FS_TRY(check_launch(ctx, "fill"));
 	}
 	auto fold_and_residual = [&]() -> int {
-		k_rel_fold<<<G, kThreads, 0, ctx->stream>>>(n, (double *)x->d, xs);
+		k_rel_fold<<<G, kThreads, 0, ctx->stream>>>(n, (double *)x->d, xs, fold);
 		FS_TRY(check_launch(ctx, "fold"));
 		return launch_spmv<double, false, false>(
 			ctx, s->A, s->A->val, (const double *)x->d, nullptr,
@@ -1986,9 +2060,9 @@ static int bicgstab_apply_reliable(Solver *s, Vec *b, Vec *x, fs_solve_info *inf
 	int64_t seen = 0;
 	const int k = k_default(s) > 1 ? k_default(s) : 32;
 	BiArgs args{b, x, k};
-	GraphKey key{b->d, x->d, 400 + k * 2 + PK};
+	GraphKey key{b->d, x->d, 400 + k * 4 + PK};
 	while (!s->hst->done && !user_stop) {
-		FS_TRY(graph_run(s, key, PK ? bi_body32<1> : bi_body32<0>, &args));
+		FS_TRY(graph_run(s, key, PK == 2 ? bi_body32<2> : PK ? bi_body32<1> : bi_body32<0>, &args));
 		FS_TRY(read_state(s));
 		if (s->hst->flags & KF_RELIABLE) {
 			FS_TRY(fold_and_residual());
@@ -2018,7 +2092,7 @@ static int bicgstab_apply_reliable(Solver *s, Vec *b, Vec *x, fs_solve_info *inf
 			seen = nh;
 		}
 	}
-	k_rel_fold<<<G, kThreads, 0, ctx->stream>>>(n, (double *)x->d, xs);
+	k_rel_fold<<<G, kThreads, 0, ctx->stream>>>(n, (double *)x->d, xs, fold);
 	FS_TRY(check_launch(ctx, "fold"));
 	FS_TRY(read_state(s));
 	KState &h = *s->hst;

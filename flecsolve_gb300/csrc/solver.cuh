@@ -100,6 +100,8 @@ struct Solver {
 	int64_t n = 0;
 	// work storage (FP64 and FP32 blocks, allocated on first apply)
 	std::vector<void *> bufs;
+	float *scaled = nullptr;  // mixed BiCGSTAB: column-scaled grid storage (on first use)
+	size_t scaled_len = 0;
 	double *w64[12] = {};
 	float *w32[12] = {};
 	double *basis = nullptr;          // GMRES: (m + 1) x n, column j contiguous

@@ -62,6 +62,7 @@ spmv_grid_kernel(CsrGrid<V> A, G g_in, Epi epi) {
 	const int nstep = (nseg + kGridThreads - 1) / kGridThreads;
 	const int segs_per_line = A.nx / W;
 	const int64_t nxy = (int64_t)A.nx * A.ny;
+	const unsigned long long once = once_policy();
 	const bool has_y = A.K >= 2, has_z = A.K >= 3;
 	const V *__restrict__ D = A.S;
 	const V *__restrict__ U1 = A.S + A.ld;
@@ -91,11 +92,17 @@ spmv_grid_kernel(CsrGrid<V> A, G g_in, Epi epi) {
 		V d[W], u1[W], u2[W], u3[W], u2m[W], u3m[W], l1[W];
 		V x[W], xmy[W], xpy[W], xmz[W], xpz[W];
 		V u1m = V(0), xm1 = V(0), xp1 = V(0);
-		ld_vec16(D + r0, d);
-		ld_vec16(U1 + r0, u1);
+		if constexpr (GEN) {
+			ld_vec16_once(D + r0, d, once);
+			ld_vec16_once(U1 + r0, u1, once);
+		}
+		else {
+			ld_vec16(D + r0, d);
+			ld_vec16(U1 + r0, u1);
+		}
 		g.at_vec(r0, x);
 		if constexpr (GEN)
-			ld_vec16(L1 + r0, l1);
+			ld_vec16_once(L1 + r0, l1, once);
 		if (lo_x) {
 			if constexpr (!GEN)
 				u1m = __ldg(U1 + r0 - 1);
@@ -104,10 +111,13 @@ spmv_grid_kernel(CsrGrid<V> A, G g_in, Epi epi) {
 		if (hi_x)
 			xp1 = g.at(r0 + W);
 		if (has_y) {
-			ld_vec16(U2 + r0, u2);
+			if constexpr (GEN)
+				ld_vec16_once(U2 + r0, u2, once);
+			else
+				ld_vec16(U2 + r0, u2);
 			if (lo_y) {
 				if constexpr (GEN)
-					ld_vec16(L2 + r0, u2m);
+					ld_vec16_once(L2 + r0, u2m, once);
 				else
 					ld_vec16(U2 + r0 - A.nx, u2m);
 				g.at_vec(r0 - A.nx, xmy);
@@ -116,10 +126,13 @@ spmv_grid_kernel(CsrGrid<V> A, G g_in, Epi epi) {
 				g.at_vec(r0 + A.nx, xpy);
 		}
 		if (has_z) {
-			ld_vec16(U3 + r0, u3);
+			if constexpr (GEN)
+				ld_vec16_once(U3 + r0, u3, once);
+			else
+				ld_vec16(U3 + r0, u3);
 			if (lo_z) {
 				if constexpr (GEN)
-					ld_vec16(L3 + r0, u3m);
+					ld_vec16_once(L3 + r0, u3m, once);
 				else
 					ld_vec16(U3 + (r0 - nxy), u3m);
 				g.at_vec((int)(r0 - nxy), xmz);
@@ -193,8 +206,10 @@ inline const double *gen_vals<double>(const Csr *A) { return A->gen64; }
 template<>
 inline const float *gen_vals<float>(const Csr *A) { return A->gen32; }
 
+// `vals`: other values in A's storage
 template<class V, bool EXACT, bool GEN, class G, class Epi>
-static inline int launch_spmv_grid(Ctx *ctx, const Csr *A, const G &g, const Epi &epi) {
+static inline int launch_spmv_grid(Ctx *ctx, const Csr *A, const G &g, const Epi &epi,
+                                   const V *vals = nullptr) {
 	static int per_sm = 0;  // resident CTAs per SM of this instantiation
 	constexpr int W = 16 / (int)sizeof(V);
 	auto kern = spmv_grid_kernel<V, EXACT, GEN, G, Epi>;
@@ -211,7 +226,7 @@ static inline int launch_spmv_grid(Ctx *ctx, const Csr *A, const G &g, const Epi
 	const int chunk = nstep >= kGridChunk * resident ? kGridChunk : 1;
 	const int nchunk = (nstep + chunk - 1) / chunk;
 	const int grid = std::max(1, std::min(nchunk, resident));
-	CsrGrid<V> d{GEN ? gen_vals<V>(A) : sym_vals<V>(A), A->sym_ld, (int)A->nrows, A->grid_nx,
+	CsrGrid<V> d{vals ? vals : GEN ? gen_vals<V>(A) : sym_vals<V>(A), A->sym_ld, (int)A->nrows, A->grid_nx,
 	             A->grid_ny, A->grid_nz, A->nsym, chunk};
 	return check_launch_rc(ctx, launch_pdl(ctx->stream, kern, grid, kGridThreads, 0, d, g, epi),
 	                       GEN ? "spmv (grid stencil, general storage)"
