@@ -265,19 +265,88 @@ __device__ void finish_step_warp(GmState *g, KState *st, double *hist, double *c
 	__syncwarp();
 }
 
-// gmres.hh:333-348, nr = k - 1
-__device__ void back_solve(GmState *g) {
-	const int nr = g->k - 1;
-	if (nr < 0)
-		return;
-	const int ld = g->ld;
-	g->dy[nr] = g->dw[nr] / g->H[nr + ld * nr];
-	for (int k = nr - 1; k >= 0; k--) {
-		g->dy[k] = g->dw[k];
-		for (int i = k + 1; i <= nr; i++)
-			g->dy[k] -= g->H[k + ld * i] * g->dy[i];
-		g->dy[k] = g->dy[k] / g->H[k + ld * k];
+// gmres.hh:333-348, nr = k - 1, by one warp: a lane holds the right-hand side
+// of rows lane, lane + 32, ..; once y_j is known every row above takes H(i, j)
+// y_j off, a product for all rows at once (17 us at nr = 29 where one thread's
+// nr^2 / 2 products and divisions took 80).  The division by the diagonal is a
+// product with its reciprocal, corrected (res_quotient).
+template<int Q>
+__device__ __forceinline__ void back_solve_rows(GmState *g) {
+	const int nr = g->k - 1, ld = g->ld, lane = threadIdx.x & 31;
+	double w[Q], d[Q], y[Q];
+	bool safe = true;  // the correction's residual is exact (res_quotient)
+#pragma unroll
+	for (int q = 0; q < Q; ++q) {
+		const int r = q * 32 + lane;
+		w[q] = r <= nr ? g->dw[r] : 0.0;
+		d[q] = r <= nr ? g->H[r + ld * r] : 1.0;
+		y[q] = 1.0 / d[q];
+		const double m = fabs(d[q]);
+		safe = safe && m > 0x1p-400 && m < 0x1p400;
 	}
+	safe = __all_sync(0xffffffffu, safe);
+	// the columns right to left, each loaded one step ahead
+	double h[Q], hn[Q];
+	auto load = [&](int j, double (&o)[Q]) {
+#pragma unroll
+		for (int q = 0; q < Q; ++q) {
+			const int r = q * 32 + lane;
+			o[q] = r < j ? g->H[r + ld * j] : 0.0;
+		}
+	};
+	load(nr, h);
+#pragma unroll 1
+	for (int j = nr; j >= 0; --j) {
+		load(j > 0 ? j - 1 : 0, hn);
+		double mine = 0.0;
+#pragma unroll
+		for (int q = 0; q < Q; ++q)
+			if (Q == 1 || q == j >> 5) {
+				const double t = w[q] * y[q], m = fabs(t);
+				mine = fma(fma(-t, d[q], w[q]), y[q], t);
+				if (lane == (j & 31) && (!safe || !(m > 0x1p-400 && m < 0x1p400)))
+					mine = w[q] / d[q];
+			}
+		const double v = __shfl_sync(0xffffffffu, mine, j & 31);
+#pragma unroll
+		for (int q = 0; q < Q; ++q) {
+			const int r = q * 32 + lane;
+			if (r == j)
+				g->dy[j] = v;
+			w[q] = fma(-h[q], v, w[q]);  // h = 0 in rows j and below
+			h[q] = hn[q];
+		}
+	}
+}
+
+__device__ void back_solve_warp(GmState *g) {
+	if (g->k > 32)
+		back_solve_rows<(kGmMaxDim + 32) / 32>(g);
+	else if (g->k > 0)
+		back_solve_rows<1>(g);
+}
+
+// (double)v of a normal number or zero in integer operations: the conversion
+// takes the FP64 pipe as long as an FMA does
+__device__ __forceinline__ double widen(float v) {
+	const unsigned b = __float_as_uint(v), a = b & 0x7fffffffu;
+	return __hiloint2double((int)((a ? (a >> 3) + 0x38000000u : 0u) | (b & 0x80000000u)), (int)(a << 29));
+}
+__device__ __forceinline__ bool widens(float v) {
+	const unsigned a = __float_as_uint(v) & 0x7fffffffu;
+	return a - 1u >= 0x7fffffu && a < 0x7f800000u;  // not subnormal, finite
+}
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ bool widens(double) { return true; }
+
+// z + sum_u c[u] v[u] with conversions (its own function: in line, the compiler
+// converts on both sides of the branch that leads here)
+template<int N, class T>
+__device__ __noinline__ double fma_converted(const double *c, const T (&v)[N], double z) {
+#pragma unroll 1
+	for (int u = 0; u < N; ++u)
+		z = fma(c[u], (double)v[u], z);
+	return z;
 }
 
 // ------------------------------------------------------------- kernels --
@@ -514,12 +583,14 @@ template<bool GATED>
 __global__ void k_gm_backsolve(GmState *g, const KState *st) {
 	if (GATED && !restart_pending(st))
 		return;
-	back_solve(g);
+	back_solve_warp(g);
 }
 
 // correct (gmres.hh:244-263) with nr = k - 1: right: z = sum_i dy_i V_i
 // accumulated left to right, x += 1.0 * P z; left: x += dy_i V_i in order.
-// x and the accumulation are FP64 for either basis type.
+// x and the accumulation are FP64 for either basis type.  Bound: the FP64 pipe,
+// an FMA a row and column (30 columns of 96^3: 111 us with converted FP32
+// entries, 67 with widen, 44 at the pipe's rate).
 template<bool GATED, class T>
 __global__ void __launch_bounds__(kT)
 k_gm_correct(int64_t n, const T *__restrict__ V, int64_t ld, const GmState *g,
@@ -533,20 +604,38 @@ k_gm_correct(int64_t n, const T *__restrict__ V, int64_t ld, const GmState *g,
 	for (int j = threadIdx.x; j <= nr; j += blockDim.x)
 		dy[j] = g->dy[j];
 	__syncthreads();
+	// eight columns' loads in flight
+	auto combine = [&](int64_t i, double z) {
+		int j = 0;
+		for (; j + 8 <= nr + 1; j += 8) {
+			T v[8];
+#pragma unroll
+			for (int u = 0; u < 8; ++u)
+				v[u] = V[(size_t)(j + u) * ld + i];
+			bool fast = true;
+#pragma unroll
+			for (int u = 0; u < 8; ++u)
+				fast = fast && widens(v[u]);
+			if (fast) {
+#pragma unroll
+				for (int u = 0; u < 8; ++u)
+					z = fma(dy[j + u], widen(v[u]), z);
+			}
+			else
+				z = fma_converted(dy + j, v, z);
+		}
+		for (; j <= nr; ++j)
+			z = fma(dy[j], (double)V[(size_t)j * ld + i], z);
+		return z;
+	};
 	FOR_EACH(i, n) {
 		if (right) {
-			double z = 0.0;
-			for (int j = 0; j <= nr; ++j)
-				z = fma(dy[j], (double)V[(size_t)j * ld + i], z);
+			const double z = combine(i, 0.0);
 			const double pz = dinv ? dinv[i] * z : z;
 			x[i] = fma(1.0, pz, x[i]);
 		}
-		else {
-			double xi = x[i];
-			for (int j = 0; j <= nr; ++j)
-				xi = fma(dy[j], (double)V[(size_t)j * ld + i], xi);
-			x[i] = xi;
-		}
+		else
+			x[i] = combine(i, x[i]);
 	}
 }
 
@@ -791,9 +880,9 @@ int gm_body(Solver *s, void *a) {
 			k_gm_mixed_cycle_end<<<1, 1, 0, ctx->stream>>>(s->st);
 			FS_TRY(check_launch(ctx, "gmres cycle end"));
 		}
-		k_gm_backsolve<true><<<1, 1, 0, ctx->stream>>>(gm_state(s), s->st);
+		k_gm_backsolve<true><<<1, 32, 0, ctx->stream>>>(gm_state(s), s->st);
 		FS_TRY(check_launch(ctx, "gmres backsolve"));
-		k_gm_correct<true, T><<<red_grid(ctx, n), kT, 0, ctx->stream>>>(
+		k_gm_correct<true, T><<<grid_for(ctx, n, kT, 1), kT, 0, ctx->stream>>>(
 			n, (const T *)s->basis, gm_ld(s), gm_state(s), s->dinv64(), (double *)ga->x->d,
 			right ? 1 : 0, s->st);
 		FS_TRY(check_launch(ctx, "gmres correct"));
@@ -970,9 +1059,9 @@ int gmres_run(Solver *s, Vec *b, Vec *x, fs_solve_info *info, bool mixed) {
 	if (!mixed || user_stop) {
 		// final correction with the current k (gmres.hh:228-233); in mixed
 		// mode every cycle was already folded into x by its tail
-		k_gm_backsolve<false><<<1, 1, 0, ctx->stream>>>(g, s->st);
+		k_gm_backsolve<false><<<1, 32, 0, ctx->stream>>>(g, s->st);
 		FS_TRY(check_launch(ctx, "gmres backsolve"));
-		k_gm_correct<false, T><<<G, kT, 0, ctx->stream>>>(n, (const T *)s->basis, ld, g, s->dinv64(),
+		k_gm_correct<false, T><<<grid_for(ctx, n, kT, 1), kT, 0, ctx->stream>>>(n, (const T *)s->basis, ld, g, s->dinv64(),
 		                                                  (double *)x->d, right ? 1 : 0, s->st);
 		FS_TRY(check_launch(ctx, "gmres correct"));
 	}

@@ -23,7 +23,7 @@
 //           last CTA forms r = sqrt(alpha - s^T s), finishes Hessenberg
 //           column k - 1 (its tentative entries + s, and r below them:
 //           M q_{k-1} = Q (h_{k-1} + s) + r q_k), then tau = q_k^T w =
-//           (gamma - s^T t) / r and the tentative column k,
+//           (gamma - s^T t) / r; pass 5's extra warp the tentative column k,
 //           h_k = Q_k^T M q_k = ([t; tau] - H s) / r, from the Arnoldi
 //           relation M Q = Q_k H;
 //   pass 5: q_k = (u_k - Q s) / r over column k, and the next candidate
@@ -211,24 +211,42 @@ __device__ __forceinline__ void staged_block_sum(const E (&acc)[NA], int nv, dou
 	__syncthreads();
 }
 
-// last CTA: out[j] = sum over CTAs of part[b * nv + j], j < nv <= 32.  Warp
-// c sums the CTAs c, c + kOWarps, ... in order (lane j: value j, so a warp
-// reads contiguous partials), then the kOWarps sums are added in order.
-__device__ __forceinline__ void staged_fold(const double *part, int nv, double *out, double *sh) {
-	const int j = threadIdx.x & 31, c = threadIdx.x >> 5;
-	double t = 0.0;
-	if (j < nv)
-		for (unsigned b = c; b < gridDim.x; b += kOWarps)
-			t += __ldcg(part + (size_t)b * nv + j);
-	__syncthreads();  // sh was used by the CTA's own sum
-	sh[c * 32 + j] = t;
+// The last CTA's sums over the CTAs of NP sets of partials, nv <= 32 values
+// each: out[32 k + j] = sum over b of part[k][b nv + j].  Warp c takes the CTAs
+// c, c + kOWarps, ... (lane j: value j, so a warp reads contiguous partials),
+// then the kOWarps sums are added, both in order.  Every load is in flight
+// before the first add, both sets: pass 4 takes 17.7 / 20.3 / 24.5 / 28.7 us at
+// up to 8 / 16 / 24 / 32 vectors of 96^3, where one set after the other in
+// batches of four loads took 19.2 / 22.4 / 26.6 / 31.3.  Every thread calls it.
+template<int NP>
+__device__ __forceinline__ void staged_fold(const double *const (&part)[NP], int nv, double *out,
+                                            unsigned char *scratch) {
+	constexpr int B = (kResMaxG + kOWarps - 1) / kOWarps;  // partials a lane holds at most
+	double *sh = reinterpret_cast<double *>(scratch);
+	const int j = threadIdx.x & 31, c = threadIdx.x >> 5, G = (int)gridDim.x;
+	double v[NP][B];
+#pragma unroll
+	for (int k = 0; k < NP; ++k)
+#pragma unroll
+		for (int i = 0; i < B; ++i) {
+			const int b = c + i * kOWarps;
+			v[k][i] = j < nv && b < G ? __ldcg(part[k] + (size_t)b * nv + j) : 0.0;
+		}
+#pragma unroll
+	for (int k = 0; k < NP; ++k) {
+		double t = v[k][0];
+#pragma unroll
+		for (int i = 1; i < B; ++i)
+			t += v[k][i];
+		sh[(k * kOWarps + c) * 32 + j] = t;
+	}
 	__syncthreads();
-	if ((int)threadIdx.x < nv) {
-		double s = 0.0;
+	if (c < NP && j < nv) {
+		double t = 0.0;
 #pragma unroll
 		for (int w = 0; w < kOWarps; ++w)
-			s += sh[w * 32 + threadIdx.x];
-		out[threadIdx.x] = s;
+			t += sh[(c * kOWarps + w) * 32 + j];
+		out[32 * c + j] = t;
 	}
 	__syncthreads();
 }
@@ -242,6 +260,23 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
 		" [%0], [%1, {%2, %3}], [%4];\n" ::"r"(smem_addr(dst)),
 		"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(smem_addr(bar))
 		: "memory");
+}
+
+// The tentative column k of the delayed form, ([t; tau] - H s) / r over rows
+// 0..k, by one warp: row i in lane i (s, t, tau and r as pass 4 left them)
+__device__ __forceinline__ void tentative_column(GmState *g, int k) {
+	const int i = threadIdx.x & 31;
+	const double r = g->dg_r, rinv = r != 0.0 ? 1.0 / r : 1.0;
+	const double rhs = i < k ? g->h2[i] : g->dg_tau;
+	double d = 0.0;
+	if (i <= k) {
+#pragma unroll 8
+		for (int j = 0; j < k; ++j) {
+			const double h = j + 1 >= i ? g->Hr[i + kGmDelayedCols * j] : 0.0;
+			d = ::fma(h, g->h1[j], d);
+		}
+		g->Hr[i + kGmDelayedCols * k] = (rhs - d) * rinv;
+	}
 }
 
 template<class T, int NA, int PASS>
@@ -437,10 +472,14 @@ k_gm_staged(OrthoArgs<T> a, const __grid_constant__ BasisMaps maps) {
 		}
 	}
 	if constexpr (PASS == 5) {
-		// the rotations, the estimate and the stop test of column k - 1,
-		// which pass 4 finished, by a warp of its own beside the update
-		if (warp == kOWarps && blockIdx.x == 0 && kp1 > 1)
-			finish_step_warp(a.g, a.st, a.hist, sh);
+		// by a warp of its own beside the update: the tentative column k for the
+		// next step's pass 4, then the rotations, the estimate and the stop test
+		// of column k - 1, which pass 4 finished
+		if (warp == kOWarps && blockIdx.x == 0) {
+			tentative_column(a.g, kp1 - 1);
+			if (kp1 > 1)
+				finish_step_warp(a.g, a.st, a.hist, sh);
+		}
 	}
 	if constexpr (PASS == 4 || PASS == 6) {
 		// pass 4: t and gamma (kp1 values, the first half of the consumers),
@@ -451,18 +490,18 @@ k_gm_staged(OrthoArgs<T> a, const __grid_constant__ BasisMaps maps) {
 		if (last_block(a.counter)) {
 			GmState *g = a.g;
 			const int k = kp1 - 1, ldh = g->ld;
-			double *Hs = reinterpret_cast<double *>(smem_raw);  // H before the rotations, k columns
 			if constexpr (PASS == 4) {
-				for (int i = tid; i < kGmDelayedCols * k; i += blockDim.x)
-					Hs[i] = g->Hr[i];
+				const double *const parts[2] = {a.part, part2};
+				staged_fold<2>(parts, kp1, folded, smem_raw);
 			}
-			staged_fold(a.part, kp1, folded, sh);
-			if constexpr (PASS == 4)
-				staged_fold(part2, kp1, folded + 32, sh);
+			else {
+				const double *const parts[1] = {a.part};
+				staged_fold<1>(parts, kp1, folded, smem_raw);
+			}
 			const double *s = PASS == 4 ? folded + 32 : folded;
 			const double *t = folded;
 			// s's and s't, a warp each
-			__shared__ double dots[3];
+			__shared__ double dots[2];
 			if (warp < 2) {
 				double d = 0.0;
 				if (lane < k)
@@ -480,28 +519,22 @@ k_gm_staged(OrthoArgs<T> a, const __grid_constant__ BasisMaps maps) {
 				if (lane == 0) {
 					dots[0] = r;
 					dots[1] = PASS == 4 ? (t[k] - dots[1]) * rinv : 0.0;
-					dots[2] = rinv;
 				}
 			}
 			__syncthreads();
-			const double r = dots[0], rinv = dots[2];
+			const double r = dots[0];
 			if (k > 0) {
 				// column k - 1 is final: its tentative entries + s, r below
 				const int c = k - 1;
 				if (tid < k) {
-					const double hv = (PASS == 4 ? Hs[tid + kGmDelayedCols * c]
-					                             : g->Hr[tid + kGmDelayedCols * c]) + s[tid];
+					const double hv = g->Hr[tid + kGmDelayedCols * c] + s[tid];
 					g->Hr[tid + kGmDelayedCols * c] = hv;
 					g->H[tid + ldh * c] = hv;
-					if constexpr (PASS == 4)
-						Hs[tid + kGmDelayedCols * c] = hv;
 				}
 				if (tid == 0) {
 					g->Hr[k + kGmDelayedCols * c] = r;
 					g->H[k + ldh * c] = r;
 					g->vnorm = r;
-					if constexpr (PASS == 4)
-						Hs[k + kGmDelayedCols * c] = r;
 				}
 				__syncthreads();
 				if constexpr (PASS == 6) {
@@ -510,29 +543,12 @@ k_gm_staged(OrthoArgs<T> a, const __grid_constant__ BasisMaps maps) {
 				}
 			}
 			if constexpr (PASS == 4) {
-				const double tau_k = dots[1];
-				// tentative column k: ([t; tau] - H s) / r over rows 0..k: row
-				// i in lane i, the k products split over the warps
-				double d = 0.0;
-				if (lane <= k)
-					for (int j = warp; j < k; j += kOWarps)
-						if (j + 1 >= lane)
-							d = ::fma(Hs[lane + kGmDelayedCols * j], s[j], d);
-				sh[warp * 32 + lane] = d;
-				__syncthreads();
-				if (tid <= k) {
-					double hs_i = sh[tid];
-#pragma unroll
-					for (int w = 1; w < kOWarps; ++w)
-						hs_i += sh[w * 32 + tid];
-					g->Hr[tid + kGmDelayedCols * k] = ((tid < k ? t[tid] : tau_k) - hs_i) * rinv;
-				}
 				if (tid < k) {
 					g->h1[tid] = s[tid];
 					g->h2[tid] = t[tid];
 				}
 				if (tid == 0) {
-					g->dg_tau = tau_k;
+					g->dg_tau = dots[1];
 					g->dg_r = r;
 				}
 			}
@@ -550,7 +566,8 @@ k_gm_staged(OrthoArgs<T> a, const __grid_constant__ BasisMaps maps) {
 		const int nv = PASS == 2 ? kp1 + 1 : kp1;
 		staged_block_sum<E, NS, false>(vals, nv, a.part, nullptr, smem_raw);
 		if (last_block(a.counter)) {
-			staged_fold(a.part, nv, folded, sh);
+			const double *const parts[1] = {a.part};
+			staged_fold<1>(parts, nv, folded, smem_raw);
 			GmState *g = a.g;
 			if constexpr (PASS == 1) {
 				if (tid < kp1)
@@ -592,7 +609,7 @@ int launch_staged(Ctx *ctx, const OrthoArgs<T> &a, const BasisMaps &maps) {
 			               kOSmemBudget + 128);
 		ready = true;
 	}
-	return check_launch_rc(ctx, launch_pdl(ctx->stream, kern, ctx->sms, kOBlock<PASS>, smem, a, maps),
+	return check_launch_rc(ctx, launch_pdl(ctx->stream, kern, std::min(ctx->sms, kResMaxG), kOBlock<PASS>, smem, a, maps),
 	                       "gmres staged orthogonalisation");
 }
 
