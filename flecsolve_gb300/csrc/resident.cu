@@ -48,6 +48,7 @@ k_cg_resident(ResCg a) {
 	struct Scalars {
 		double tol, tol2, rho, rho_inv, rho_old, pap, rr, rr0, rhs_norm, sol0, beta, xx;
 		int it, status, info_iters, flags;
+		int turn;  // CTA that keeps the next entry of the history
 	};
 	__shared__ Scalars z;
 	ResTeam tm;
@@ -169,9 +170,10 @@ k_cg_resident(ResCg a) {
 		if (tid == 32)
 			z.rho_inv = 1.0 / z.rho;  // for beta; this warp has no message to carry
 		if (tid == 0) {
-			sh.bc[0] = z.rho / pap;
+			sh.bc[0] = res_divide(z.rho, pap);
 			z.pap = pap;
-			if (!(pap > 0.0))
+			const long long sign = __double_as_longlong(pap);
+			if (!(sign > 0 && sign <= 0x7ff0000000000000ll))  // !(pap > 0)
 				z.flags |= KF_NEG_CURVATURE;
 		}
 		if (!(alive = tm.done()))
@@ -207,16 +209,19 @@ k_cg_resident(ResCg a) {
 			z.rr = rr;
 			// each CTA keeps every gridDim-th entry of the history, its root
 			// taken at the end
-			if (it <= a.hist_cap && (unsigned)(it - 1) % gridDim.x == blockIdx.x)
+			const int turn = z.turn;
+			if (it <= a.hist_cap && turn == (int)blockIdx.x)
 				a.hist[it - 1] = rr;
-			if (!isfinite(rr))
+			z.turn = turn + 1 < (int)gridDim.x ? turn + 1 : 0;
+			const bool finite = res_finite(rr);
+			if (!finite)
 				z.flags |= KF_NONFINITE;
-			if (rr <= z.tol2) {
+			if (finite && res_below(rr, z.tol2)) {
 				sh.stop = 1;
 				z.status = FS_CONVERGED_RTOL;
 				z.info_iters = it;
 			}
-			else if (it >= a.maxiter || (z.flags & KF_NONFINITE)) {
+			else if (it >= a.maxiter || !finite) {
 				sh.stop = 1;
 				z.status = FS_DIVERGED_ITERS;
 			}

@@ -473,6 +473,15 @@ __device__ __forceinline__ double res_threshold(double tol) {
 	return t;
 }
 
+__device__ __forceinline__ int res_exponent(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+__device__ __forceinline__ bool res_finite(double v) { return res_exponent(v) != 0x7ff; }
+// s <= t for a sum of squares s that is finite (a comparison is an FP64
+// operation; non-negative doubles compare as integers, and a negative t is
+// below all of them)
+__device__ __forceinline__ bool res_below(double s, double t) {
+	return __double_as_longlong(s) <= __double_as_longlong(t);
+}
+
 // a / b, correctly rounded, from y = 1 / b correctly rounded (Markstein 1990:
 // the residual of a y corrects it); three dependent operations after a is
 // known where a division takes 561 cycles.  Outside the range where the
@@ -480,10 +489,28 @@ __device__ __forceinline__ double res_threshold(double tol) {
 __device__ __forceinline__ double res_quotient(double a, double b, double y) {
 	const double q = a * y;
 	const double r = fma(fma(-q, b, a), y, q);
-	const double m = fabs(a), n = fabs(b);
-	const bool safe = m > 0x1p-900 && m < 0x1p900 && n > 0x1p-900 && n < 0x1p900 && fabs(q) > 0x1p-900 &&
-	                  fabs(q) < 0x1p900;
+	const bool safe = (unsigned)(res_exponent(a) - 123) < 1800u && (unsigned)(res_exponent(b) - 123) < 1800u &&
+	                  (unsigned)(res_exponent(q) - 123) < 1800u;
 	return safe ? r : a / b;
+}
+
+// a / b to half a unit in the last place and 2^-37 of one: b's reciprocal from
+// the FP32 one of its leading bits and one Newton step (2^-45), the quotient's
+// residual as above.  Five dependent FP64 operations on the path of a sum that
+// everything waits for; the division takes ten.
+__device__ __forceinline__ double res_divide(double a, double b) {
+	const int ea = res_exponent(a), eb = res_exponent(b), hi = __double2hiint(b);
+	if ((unsigned)(ea - 523) >= 1000u || (unsigned)(eb - 523) >= 1000u)
+		return a / b;
+	const float m = __int_as_float(0x3f800000 | (int)((unsigned)hi << 3 & 0x7fffff) |
+	                               (int)((unsigned)__double2loint(b) >> 29));
+	const unsigned f = __float_as_uint(__frcp_rn(m));  // 2^-1 .. 1
+	const unsigned e = (f >> 23) + (unsigned)(1919 - eb);  // biased; 1 / 2^(eb - 1023)
+	const double y0 = __hiloint2double((int)(((unsigned)hi & 0x80000000u) | e << 20 | (f >> 3 & 0xfffffu)),
+	                                   (int)(f << 29));
+	const double y = fma(fma(-b, y0, 1.0), y0, y0);
+	const double q = a * y;
+	return fma(fma(-q, b, a), y, q);
 }
 
 // the payload of a packet that had not arrived at the first look (its own

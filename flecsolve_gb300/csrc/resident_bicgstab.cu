@@ -41,6 +41,7 @@ k_bi_resident(ResBi a) {
 		double tol, tol2, rtol2, rho, rho_inv, rho_old, alpha, omega, ao, beta, rr, rr0, ss, rhs_norm,
 			sol0, rt_norm, rt_eps, xx;  // tol2, rtol2, rt_eps: res_threshold of the tests
 		int it, nhist, status, info_iters, flags, restarts;
+		int turn;  // CTA that keeps the next entry of the history
 		int what;  // thread 0's verdict: 1 stop, 2 early exit, 3 restart
 	};
 	__shared__ Scalars z;
@@ -184,7 +185,7 @@ k_bi_resident(ResBi a) {
 			});
 		const double rv = tm.grid_sum<1, false>(s1);
 		if (tid == 0) {
-			z.alpha = z.rho / rv;
+			z.alpha = res_divide(z.rho, rv);
 			if (!(rv != 0.0)) {
 				z.flags |= KF_ALPHA_ZERO;
 				z.what = 1;
@@ -235,7 +236,7 @@ k_bi_resident(ResBi a) {
 				z.info_iters = z.it;
 				z.status = FS_CONVERGED_RTOL;
 			}
-			z.omega = sh.bc[1] == 0.0 ? 0.0 : sh.bc[2] / sh.bc[1];
+			z.omega = sh.bc[1] == 0.0 ? 0.0 : res_divide(sh.bc[2], sh.bc[1]);
 		}
 		__syncthreads();
 		if (z.what == 2) {
@@ -280,13 +281,16 @@ k_bi_resident(ResBi a) {
 			z.rr = rr;
 			// each CTA keeps every gridDim-th entry of the history, its root
 			// taken at the end
-			if (z.nhist < a.hist_cap && (unsigned)z.nhist % gridDim.x == blockIdx.x)
+			const int turn = z.turn;
+			if (z.nhist < a.hist_cap && turn == (int)blockIdx.x)
 				a.hist[z.nhist] = rr;
+			z.turn = turn + 1 < (int)gridDim.x ? turn + 1 : 0;
 			z.nhist += 1;
-			if (!isfinite(rr))
+			const bool finite = res_finite(rr);
+			if (!finite)
 				z.flags |= KF_NONFINITE;
 			int what = 0;
-			if (rr <= z.tol2) {
+			if (finite && res_below(rr, z.tol2)) {
 				what = 1;
 				z.status = FS_CONVERGED_RTOL;
 				z.info_iters = it + 1;
@@ -300,7 +304,7 @@ k_bi_resident(ResBi a) {
 			z.rho = rho;
 			z.it = it + 1;
 			if (!what) {
-				if (it + 1 >= a.maxiter || (z.flags & KF_NONFINITE)) {
+				if (it + 1 >= a.maxiter || !finite) {
 					what = 1;
 					z.status = FS_DIVERGED_ITERS;
 				}
