@@ -7,6 +7,9 @@
 //    passes over V -- (1) h = V^T v; (2) v -= V h and h2 = V^T v in the same
 //    pass; (3) v -= V h2 with ||v||^2 -- so a step costs 3 reductions instead
 //    of the k + 2 of modified Gram-Schmidt.
+//  * DCGS2: CGS2 with the reorthogonalisation delayed to the next step
+//    (gmres_staged.cuh); small grid stencils run it as one cooperative launch
+//    (resident_gmres.cu).
 //  * MGS: the reference's modified Gram-Schmidt order (gmres.hh:265-279),
 //    one fused "v -= h_{j-1} V_{j-1}; h_j = v . V_j" kernel per basis vector.
 // The Hessenberg column, the Givens rotations (Bindel, Demmel, Kahan,

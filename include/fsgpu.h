@@ -364,7 +364,9 @@ enum fs_gmres_side { FS_LEFT = 0, FS_RIGHT = 1 };
 /* GMRES orthogonalisation.  AUTO picks MGS for the FP64 basis (half the FP64
  * multiply-adds of CGS2, and the reference's order) and DCGS2 (below; CGS2
  * where DCGS2 cannot run) for the FP32 basis of FS_GMRES_MIXED: 2 passes and
- * 1 reduction per step instead of the k + 2 of MGS.
+ * 1 reduction per step instead of the k + 2 of MGS.  On a grid-stencil operator
+ * of up to 1,000,000 rows (FS_GMRES_MIXED: 450,000) AUTO and DCGS2 run the whole
+ * solve as one cooperative launch with DCGS2 (m <= 30, no diagnostic callback).
  * DCGS2: CGS2 with each vector's reorthogonalisation delayed to the next
  * step, where it shares that step's pass of dot products (two passes over
  * the basis a step instead of three); the convergence test of a step runs
