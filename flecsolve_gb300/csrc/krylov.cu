@@ -540,12 +540,10 @@ k_bi_start(int64_t n, const V *__restrict__ res, V *__restrict__ rt, V *__restri
 	}
 }
 
-// p update (bicgstab.hh:115-122).  BACK: rows from the last to the first.
-template<class V, bool BACK = false>
+// p update (bicgstab.hh:115-122)
+template<class V>
 __global__ void k_bi_p(int64_t n, V *__restrict__ p, const V *__restrict__ v,
                        const V *__restrict__ res, const KState *st) {
-	pdl_wait();
-	pdl_trigger();
 	if (stopped(st))
 		return;
 	if (st->iter == 0) {
@@ -562,8 +560,7 @@ __global__ void k_bi_p(int64_t n, V *__restrict__ p, const V *__restrict__ v,
 			float4 *p4 = reinterpret_cast<float4 *>(p);
 			const float4 *v4 = reinterpret_cast<const float4 *>(v);
 			const float4 *r4 = reinterpret_cast<const float4 *>(res);
-			FOR_EACH(e, n4) {
-				const int64_t i = BACK ? n4 - 1 - e : e;
+			FOR_EACH(i, n4) {
 				float4 pv = p4[i];
 				const float4 vv = v4[i], rv = r4[i];
 				one(pv.x, vv.x, rv.x);
@@ -591,7 +588,6 @@ struct EpiBiV {
 	KState *st;
 	double *part;
 	unsigned *counter;
-	bool backwards = false;
 	__device__ bool skip() const { return stopped(st); }
 	template<class A>
 	__device__ void row(int r, V s, A &acc) const {
@@ -610,13 +606,11 @@ struct EpiBiV {
 };
 
 // s = res - alpha v, s_norm; early exit when s_norm < rtol (bicgstab.hh:132-143)
-template<class V, bool BACK = false>
+template<class V>
 __global__ void __launch_bounds__(kThreads)
 k_bi_s(int64_t n, V *__restrict__ s, const V *__restrict__ v, const V *__restrict__ res,
        KState *st, double *part, unsigned *counter) {
 	__shared__ double sh[128];
-	pdl_wait();
-	pdl_trigger();
 	if (stopped(st))
 		return;
 	const V a = (V)st->alpha;
@@ -632,8 +626,7 @@ k_bi_s(int64_t n, V *__restrict__ s, const V *__restrict__ v, const V *__restric
 		float4 *s4 = reinterpret_cast<float4 *>(s);
 		const float4 *v4 = reinterpret_cast<const float4 *>(v);
 		const float4 *r4 = reinterpret_cast<const float4 *>(res);
-		FOR_EACH(e, n4) {
-			const int64_t i = BACK ? n4 - 1 - e : e;
+		FOR_EACH(i, n4) {
 			float4 sv;
 			const float4 vv = v4[i], rv = r4[i];
 			one(sv.x, vv.x, rv.x);
@@ -672,7 +665,6 @@ struct EpiBiT {
 	KState *st;
 	double *part;
 	unsigned *counter;
-	bool backwards = false;
 	__device__ bool skip() const { return stopped(st) || (st->flags & KF_EARLY); }
 	template<class A>
 	__device__ void row(int r, V val, A &acc) const {
@@ -695,15 +687,13 @@ struct EpiBiT {
 // raises KF_RELIABLE with the reason in aux[3] (0 drop, 1 converged, 2 early
 // exit, 3 omega == 0, 4 maxiter) and the host replaces the residual by the
 // FP64 one before deciding.
-template<class V, int PK, bool RELY = false, bool BACK = false>
+template<class V, int PK, bool RELY = false>
 __global__ void __launch_bounds__(kThreads)
 k_bi_x(int64_t n, V *__restrict__ x, const V *__restrict__ p, const V *__restrict__ s,
        const V *__restrict__ t, V *__restrict__ res, const V *__restrict__ rt,
        const V *__restrict__ dinv, KState *st, double *part, unsigned *counter,
        double *hist) {
 	__shared__ double sh[128];
-	pdl_wait();
-	pdl_trigger();
 	if (stopped(st))
 		return;
 	const V a = (V)st->alpha;
@@ -747,8 +737,7 @@ k_bi_x(int64_t n, V *__restrict__ x, const V *__restrict__ p, const V *__restric
 		const float4 *t4 = reinterpret_cast<const float4 *>(t);
 		const float4 *q4 = reinterpret_cast<const float4 *>(rt);
 		const float4 *d4 = reinterpret_cast<const float4 *>(dinv);
-		FOR_EACH(e, n4) {
-			const int64_t i = BACK ? n4 - 1 - e : e;
+		FOR_EACH(i, n4) {
 			float4 xv = x4[i], rv;
 			const float4 pv = p4[i], sv = s4[i], tv = t4[i], qv = q4[i];
 			const float4 dv = PK ? d4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1581,6 +1570,12 @@ struct RcArgs {
 	double delta;
 };
 
+// Rows from which the passes of mixed CG alternate direction: us an iteration
+// forwards / alternating 27.6 / 27.9 at 64^3, 35.7 / 36.0 at 96^3, 75.3 / 76.0 at
+// 160^3, 127.6 / 127.2 at 200^3, 216.5 / 214.1 at 256^3.  While an iteration's 64
+// bytes a row fit twice in the L2, both orders find what the last pass left.
+constexpr int64_t kTurnRows = 6000000;
+
 template<int PK>
 static int rc_body(Solver *s, void *a) {
 	RcArgs *g = (RcArgs *)a;
@@ -1594,15 +1589,15 @@ static int rc_body(Solver *s, void *a) {
 	// what that one left in the L2: the residual pass on the SpMV's last w, the
 	// direction pass on the residual pass's last r and D^-1, the next SpMV on
 	// the direction pass's last p (a body of an odd count starts like an even
-	// one; only the first pass of the next body then misses).  256^3 diffusion,
-	// 1,465 iterations: 317.1 ms with forward passes, 313.7 ms so.
+	// one; only the first pass of the next body then misses).
+	const bool turn = n >= kTurnRows;
 	for (int k = 0; k < g->k; ++k) {
-		const bool back = k & 1;
+		const bool back = turn && (k & 1), rback = turn && !back;
 		FS_TRY(launch_spmv<float, false, false>(
 			ctx, s->A, s->A->val32, p, nullptr,
 			EpiCgAp<float>{w, p, s->st, s->part, s->counter, back}));
 		FS_TRY(check_launch_rc(ctx,
-		                       launch_pdl(ctx->stream, back ? k_rc_resid4<PK, false> : k_rc_resid4<PK, true>,
+		                       launch_pdl(ctx->stream, rback ? k_rc_resid4<PK, true> : k_rc_resid4<PK, false>,
 		                                  G4, kThreads, 0, n, r, w, dinv, s->st, s->part, s->counter,
 		                                  s->hist, g->delta),
 		                       "reliable cg update"));
@@ -1824,27 +1819,25 @@ static int bi_body64(Solver *s, void *a) {
 	const double *dinv = s->dinv64();
 	const int G = red_grid(ctx, n);
 	for (int k = 0; k < g->k; ++k) {
-		FS_TRY(check_launch_rc(ctx, launch_pdl(ctx->stream, k_bi_p<double>, G, kThreads, 0, n, p, v, res,
-		                                       (const KState *)s->st),
-		                       "bicgstab p"));
+		k_bi_p<double><<<G, kThreads, 0, ctx->stream>>>(n, p, v, res, s->st);
+		FS_TRY(check_launch(ctx, "bicgstab p"));
 		if (PK)
 			FS_TRY((launch_spmv<double, false, true>(ctx, s->A, s->A->val, p, dinv,
 			                                         EpiBiV<double>{v, rt, s->st, s->part, s->counter})));
 		else
 			FS_TRY((launch_spmv<double, false, false>(ctx, s->A, s->A->val, p, nullptr,
 			                                          EpiBiV<double>{v, rt, s->st, s->part, s->counter})));
-		FS_TRY(check_launch_rc(ctx, launch_pdl(ctx->stream, k_bi_s<double>, G, kThreads, 0, n, sv, v, res,
-		                                       s->st, s->part, s->counter),
-		                       "bicgstab s"));
+		k_bi_s<double><<<G, kThreads, 0, ctx->stream>>>(n, sv, v, res, s->st, s->part, s->counter);
+		FS_TRY(check_launch(ctx, "bicgstab s"));
 		if (PK)
 			FS_TRY((launch_spmv<double, false, true>(ctx, s->A, s->A->val, sv, dinv,
 			                                         EpiBiT<double>{t, sv, s->st, s->part, s->counter})));
 		else
 			FS_TRY((launch_spmv<double, false, false>(ctx, s->A, s->A->val, sv, nullptr,
 			                                          EpiBiT<double>{t, sv, s->st, s->part, s->counter})));
-		FS_TRY(check_launch_rc(ctx, launch_pdl(ctx->stream, k_bi_x<double, PK>, G, kThreads, 0, n, x, p,
-		                                       sv, t, res, rt, dinv, s->st, s->part, s->counter, s->hist),
-		                       "bicgstab x"));
+		k_bi_x<double, PK><<<G, kThreads, 0, ctx->stream>>>(n, x, p, sv, t, res, rt, dinv, s->st,
+		                                                   s->part, s->counter, s->hist);
+		FS_TRY(check_launch(ctx, "bicgstab x"));
 	}
 	return FS_OK;
 }
@@ -1927,9 +1920,9 @@ static int bicgstab_apply64(Solver *s, Vec *b, Vec *x, fs_solve_info *info) {
 // The general grid storage with column c scaled by D^-1(c): right Jacobi
 // preconditioning in the values, from the FP64 ones, rounded once.  Bound: HBM.
 // It takes the seven scale loads a row from both SpMVs of an iteration (54 and
-// 47 us at 192^3 with them, 51 and 45 without) and D^-1 from three passes: with
-// the passes launched ahead and walking against each other, 201 -> 170 us an
-// iteration, against 137 us of memory traffic.
+// 47 us at 192^3 with them, 51 and 45 without) and D^-1 from three passes: 201
+// -> 172 us an iteration, 162 with the values leaving the L2 first, against 137
+// us of memory traffic.
 __global__ void k_scale_cols(int n, int K, int d2, int d3, int64_t ld, const double *__restrict__ S,
                              const double *__restrict__ dinv, float *__restrict__ out) {
 	const int off[4] = {0, 1, d2, d3};
@@ -1989,29 +1982,19 @@ static int bi_body32(Solver *s, void *a) {
 		else
 			return launch_spmv<float, false, PK == 1>(ctx, s->A, s->A->val32, x, dinv, epi);
 	};
-	// the passes alternate direction, as in mixed CG
-	bool back = false;
+	// plain launches: let in early, the next pass costs the running one more
+	// than its own start (96^3: 47.9 us an iteration with programmatic launches,
+	// 42.5 without; 192^3: 161.3 and 162.0)
 	for (int k = 0; k < g->k; ++k) {
-		FS_TRY(check_launch_rc(ctx, launch_pdl(ctx->stream, back ? k_bi_p<float, true> : k_bi_p<float, false>,
-		                                       G, kThreads, 0, n, p, v, res, (const KState *)s->st),
-		                       "bicgstab p f32"));
-		back = !back;
-		FS_TRY(spmv(p, EpiBiV<float>{v, rt, s->st, s->part, s->counter, back}));
-		back = !back;
-		FS_TRY(check_launch_rc(ctx, launch_pdl(ctx->stream, back ? k_bi_s<float, true> : k_bi_s<float, false>,
-		                                       G, kThreads, 0, n, sv, v, res, s->st, s->part, s->counter),
-		                       "bicgstab s f32"));
-		back = !back;
-		FS_TRY(spmv(sv, EpiBiT<float>{t, sv, s->st, s->part, s->counter, back}));
-		back = !back;
-		constexpr int PX = PK == 1;
-		FS_TRY(check_launch_rc(ctx,
-		                       launch_pdl(ctx->stream,
-		                                  back ? k_bi_x<float, PX, true, true> : k_bi_x<float, PX, true, false>,
-		                                  G, kThreads, 0, n, xs, p, sv, t, res, rt, dinv, s->st, s->part,
-		                                  s->counter, s->hist),
-		                       "bicgstab x f32"));
-		back = !back;
+		k_bi_p<float><<<G, kThreads, 0, ctx->stream>>>(n, p, v, res, s->st);
+		FS_TRY(check_launch(ctx, "bicgstab p f32"));
+		FS_TRY(spmv(p, EpiBiV<float>{v, rt, s->st, s->part, s->counter}));
+		k_bi_s<float><<<G, kThreads, 0, ctx->stream>>>(n, sv, v, res, s->st, s->part, s->counter);
+		FS_TRY(check_launch(ctx, "bicgstab s f32"));
+		FS_TRY(spmv(sv, EpiBiT<float>{t, sv, s->st, s->part, s->counter}));
+		k_bi_x<float, PK == 1, true><<<G, kThreads, 0, ctx->stream>>>(n, xs, p, sv, t, res, rt, dinv, s->st,
+		                                                             s->part, s->counter, s->hist);
+		FS_TRY(check_launch(ctx, "bicgstab x f32"));
 	}
 	return FS_OK;
 }

@@ -192,7 +192,8 @@ __device__ __forceinline__ void ld_vec16(const double *p, double (&o)[2]) {
 
 // the same for values that a kernel reads once: not kept in the L1, first to
 // leave the L2, so that the vectors between two passes stay there instead
-// (mixed BiCGSTAB's iteration at 192^3 170.5 -> 163.7 us, at 128^3 80.8 -> 76.3)
+// (mixed BiCGSTAB's iteration at 192^3 172.7 -> 162.0 us, at 128^3 81.5 -> 76.8,
+// at 96^3, where all of it stays, 42.3 -> 42.5)
 __device__ __forceinline__ unsigned long long once_policy() {
 	unsigned long long p;
 	asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
