@@ -115,12 +115,19 @@ struct RgAcc<float> {
 };
 
 // the CTA's copy of the small state (the same in every CTA)
+//
+// A step's scalars have a slot for each parity: the Hessenberg warp reads those
+// of step k until it joins the barrier of step k + 1, while warp 0 may already
+// write those of step k + 1; step k + 2 writes after that barrier.
+struct RgStep {
+	double s[kGmDelayedCols], t[kGmDelayedCols];       // totals
+	double r, rinv, tau;
+};
 struct RgSmall {
-	double s[kGmDelayedCols], t[kGmDelayedCols];       // totals of the step
+	RgStep step[2];
 	double Hr[kGmDelayedCols * kGmDelayedCols];        // Hessenberg before the rotations
 	double H[kGmDelayedCols * kGmDelayedCols];         // and after
 	double cs[kGmDelayedCols], sn[kGmDelayedCols], dw[kGmDelayedCols + 1], dy[kGmDelayedCols];
-	double r, rinv, tau;                               // of the step
 	double bnorm, tol, rhs_norm, sol0, res0, res, beta, xx;
 	int k;                                             // finished columns
 	int it, nhist, status, info_iters, flags, restarts;
@@ -136,19 +143,19 @@ __device__ __forceinline__ void rg_bar(int threads) {
 // column c of the Hessenberg matrix is final up to the step's s and r:
 // rotations, estimate and stop tests (finish_step_warp of gmres.cu on the
 // CTA's copy; only CTA 0 writes the history)
-__device__ void rg_finish_column(RgSmall &g, int c, double *hist, int hist_cap, int maxiter, int m,
-                                 int mixed, int *flag) {
+__device__ void rg_finish_column(RgSmall &g, const RgStep &st, int c, double *hist, int hist_cap,
+                                 int maxiter, int m, int mixed, int *flag) {
 	constexpr int ld = kGmDelayedCols;
 	const int lane = threadIdx.x & 31;
 	double *col = g.H + ld * c;
 	if (lane < c + 1) {
-		const double h = g.Hr[lane + ld * c] + g.s[lane];
+		const double h = g.Hr[lane + ld * c] + st.s[lane];
 		g.Hr[lane + ld * c] = h;
 		col[lane] = h;
 	}
 	if (lane == 0) {
-		g.Hr[c + 1 + ld * c] = g.r;
-		col[c + 1] = g.r;
+		g.Hr[c + 1 + ld * c] = st.r;
+		col[c + 1] = st.r;
 	}
 	__syncwarp();
 	double x = col[0];
@@ -161,7 +168,7 @@ __device__ void rg_finish_column(RgSmall &g, int c, double *hist, int hist_cap, 
 		x = __shfl_sync(0xffffffffu, v, 1);
 	}
 	if (lane == 0) {
-		const double gg = g.r;
+		const double gg = st.r;
 		col[c] = x;
 		if (gg != 0.0) {
 			double cc, s;
@@ -387,6 +394,7 @@ k_gm_resident(ResGm<T> a) {
 		for (int k = 0;; ++k) {
 			const bool last = k == a.m;  // u_m's sums alone finish the cycle
 			const int nv = last ? k + 1 : 2 * (k + 1);
+			RgStep &st = g.step[k & 1];
 			++tm.epoch;
 			if (worker) {
 				if (!last) {
@@ -496,17 +504,17 @@ k_gm_resident(ResGm<T> a) {
 						sw += __shfl_xor_sync(0xffffffffu, sw, o);
 					}
 					if (lane <= k) {
-						g.s[lane] = q[0];
-						g.t[lane] = q[1];
+						st.s[lane] = q[0];
+						st.t[lane] = q[1];
 						hs[lane] = (T)q[0];
 						ht[lane] = (T)q[1];
 					}
 					const double r = k > 0 ? sqrt(fmax(alpha - ss, 0.0)) : 1.0;
 					const double rinv = r != 0.0 ? 1.0 / r : 1.0;
 					if (lane == 0) {
-						g.r = r;
-						g.rinv = rinv;
-						g.tau = (gamma - sw) * rinv;
+						st.r = r;
+						st.rinv = rinv;
+						st.tau = (gamma - sw) * rinv;
 					}
 				}
 			}
@@ -522,15 +530,15 @@ k_gm_resident(ResGm<T> a) {
 			}
 			if (!worker) {
 				if (k > 0)
-					rg_finish_column(g, k - 1, a.hist, a.hist_cap, a.maxiter, a.m, a.mixed,
+					rg_finish_column(g, st, k - 1, a.hist, a.hist_cap, a.maxiter, a.m, a.mixed,
 					                 &g.flag[k & 1]);
 				if (!last && lane <= k) {
 					// tentative column k: ([t; tau] - H s) / r over rows 0..k
 					double d = 0.0;
 					for (int j = 0; j < k; ++j)
 						if (j + 1 >= lane)
-							d = fma(g.Hr[lane + kGmDelayedCols * j], g.s[j], d);
-					g.Hr[lane + kGmDelayedCols * k] = ((lane < k ? g.t[lane] : g.tau) - d) * g.rinv;
+							d = fma(g.Hr[lane + kGmDelayedCols * j], st.s[j], d);
+					g.Hr[lane + kGmDelayedCols * k] = ((lane < k ? st.t[lane] : st.tau) - d) * st.rinv;
 				}
 				__syncwarp();
 			}
@@ -543,7 +551,7 @@ k_gm_resident(ResGm<T> a) {
 			if (worker) {
 				// q_k = (u_k - Q s) / r, u_{k+1} = (w - Q t - tau q_k) / r
 				T *uk = col[k], *un = col[k + 1];
-				const T inv = (T)g.rinv, tau = (T)-g.tau;
+				const T inv = (T)st.rinv, tau = (T)-st.tau;
 				tag = tm.epoch;
 				for (int c = tid; c < nch; c += ntk) {
 					T q[W], n[W];

@@ -233,3 +233,37 @@ def test_resident_bicgstab_stops(ctx):
         assert (one.status, one.iters) == (ref.status, ref.iters)
         assert h1.size == h2.size
         assert np.linalg.norm(x1 - x2) <= 1e-9 * max(np.linalg.norm(x2), 1e-30)
+
+
+@pytest.mark.parametrize("shape,dims,asym", [((12, 11, 1), 2, 0.3), ((16, 32, 1), 2, 0.0), ((48, 44, 1), 2, 0.3),
+                                             ((36, 20, 17), 3, 0.3)])
+@pytest.mark.parametrize("method,u", [("gmres", 2.0 ** -53), ("mixed_gmres", 2.0 ** -24)])
+def test_resident_gmres_estimate_is_the_true_residual(ctx, method, u, shape, dims, asym):
+    """Every Hessenberg column and rotation: stopped after k steps, the
+    estimate is the norm of b - A x_k.  A P V = V H + E with 8 + 2 (k + 1)
+    roundings an entry in SpMV and update and |A D^-1| <= 2, so the two differ by
+    at most 4 (k + 5) u (sqrt(k) |y| + estimate), |y| = |D x|; four times that
+    for the norms formed from dots.  Solves repeat bit for bit."""
+    A = _grid(*shape, dims, seed=sum(shape), asym=asym)
+    b = P.uniform(3, A.nrows)
+    M = A.to_scipy()
+    D = M.diagonal()
+    dA, vb = fs.CSR(ctx, A), fs.Vector(ctx, b)
+    assert dA.index_coding("grid") is not None
+    ns = getattr(fs, method)
+    first = None
+    for k in list(range(1, 32)) + [31, 31]:
+        s = ns.settings(use_zero_guess=True, maxiter=k, rtol=1e-30, max_krylov_dim=30, restart=True, ortho="dcgs2")
+        vx = fs.Vector(ctx, A.nrows)
+        slv = ns.solver(s, ns.make_work(vb))(fs.op.ref(dA), fs.op.jacobi)
+        slv(vb, vx)
+        h, x = slv.history(), vx.numpy()
+        assert h.size == k
+        if k < 31:
+            true = np.linalg.norm(b - M @ x)
+            bound = 16 * (k + 5) * u * (np.sqrt(k) * np.linalg.norm(D * x) + h[-1])
+            assert abs(h[-1] - true) <= bound, (k, h[-1], true, bound)
+        elif first is None:
+            first = h, x
+        else:
+            assert np.array_equal(h, first[0]) and np.array_equal(x, first[1])
