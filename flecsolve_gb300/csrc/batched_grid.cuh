@@ -196,6 +196,9 @@ k_batch_grid(BatchArgs a) {
 		return t;
 	};
 
+	// a peer's shared memory may be written once all CTAs of the cluster run
+	team_sync();
+
 	// ||b||, ||x||
 	double bnorm, res;
 	{

@@ -69,3 +69,22 @@ def test_grid_batch_special_systems(ctx):
         assert all(abs(p.iters - q.iters) <= 3 for p, q in zip(i, ref))
         assert np.isfinite(x[off[2]:]).all()
         assert np.isfinite(x[off[1]:off[2]]).all() == np.isfinite(xr[off[1]:off[2]]).all()
+
+
+def test_grid_batch_with_clusters_that_wait_for_room(ctx):
+    """Far more 15-CTA clusters than the GPU holds at once, so that clusters
+    start while others end and their CTAs start apart: every system meets its
+    tolerance, and repeated calls return the same bits."""
+    A, off, b = _batch([400] * 40)
+    S = A.to_scipy()
+    dA, vb = fs.CSR(ctx, A), fs.Vector(ctx, b)
+    xs = []
+    for _ in range(3):
+        vx = fs.Vector(ctx, A.nrows)
+        infos = fs.batch_cg(dA, off, vb, vx, maxiter=4000, rtol=1e-5)
+        assert all(i.status == "converged_rtol" for i in infos)
+        xs.append(vx.numpy())
+    r = b - S @ xs[0]
+    for lo, hi in zip(off[:-1], off[1:]):
+        assert np.linalg.norm(r[lo:hi]) <= 1e-5 * (1 + 1e-3) * np.linalg.norm(b[lo:hi])
+    assert np.array_equal(xs[0], xs[1]) and np.array_equal(xs[0], xs[2])
