@@ -124,7 +124,12 @@ struct Csr {
 	double *gen64 = nullptr;
 	float *gen32 = nullptr;
 	bool gen64_valid = false, gen32_valid = false;
-	int sym_state = -1;             // -1 not checked since the values changed, 0 no, 1 yes
+	// every lower entry equals its upper partner bit for bit: -1 not checked
+	// since the values changed, 0 no, 1 yes
+	int sym_state = -1;
+	// as many lower as upper entries and no column twice in a row: with
+	// sym_state == 1 every upper entry has its lower partner, too
+	bool sym_paired = false;
 	// FMA-mode column-id SpMV kernel per value type (0 FP64, 1 FP32): 0 row
 	// blocks, L = 4..32 lanes per row of the vector kernel, 1 the vector
 	// kernel with rows binned by length, -1 not tuned yet

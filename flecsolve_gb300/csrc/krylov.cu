@@ -2383,17 +2383,19 @@ FS_API int fs_krylov_apply(fs_solver h, fs_vec bh, fs_vec xh, fs_solve_info *inf
 
 // A^T x = b with the bound solver's method, settings and preconditioner
 // (the Jacobi diagonal of A^T is A's).  The transposed operator is a view of
-// A's CSC arrays, refreshed from A's current values on every call.
+// A's CSC arrays, refreshed from A's current values on every call, or A
+// itself when its pattern and values are symmetric.
 FS_API int fs_krylov_apply_transpose(fs_solver h, fs_vec bh, fs_vec xh, fs_solve_info *info) {
 	Solver *s = reinterpret_cast<Solver *>(h);
 	if (!ok_slv(s))
 		return FS_ERR_BAD_HANDLE;
 	Csr *A = s->A;
 	FS_TRY(reject_matrix_free(A, "transpose"));
+	cudaSetDevice(A->ctx->device);
 	// a matrix that is symmetric bit for bit is its own transpose: its own
 	// storage serves (no column view built or refreshed)
 	FS_TRY(ensure_sym(A, false));
-	if (A->sym_state == 1)
+	if (A->sym_state == 1 && A->sym_paired)
 		return fs_krylov_apply(h, bh, xh, info);
 	FS_TRY(ensure_transpose(A));
 	FS_TRY(ensure_dinv(A));

@@ -136,6 +136,26 @@ static bool sym_slots(const std::vector<int> &ptab, const std::vector<int> &plen
 	return true;
 }
 
+// Whether the rows hold as many lower as upper entries, none of them twice.
+// Lower entries with distinct upper partners are then all the upper entries'
+// partners: the pattern is its own transpose.
+static bool paired(int64_t n, const std::vector<int> &ptab, const std::vector<int> &plen, int npat,
+                   const std::vector<unsigned char> &pid) {
+	std::vector<int> net(npat, 0);  // upper less lower entries of a pattern
+	for (int p = 0; p < npat; ++p) {
+		const int *d = &ptab[(size_t)p * kPatW];
+		for (int j = 0; j < plen[p]; ++j) {
+			net[p] += (d[j] > 0) - (d[j] < 0);
+			if (std::find(d, d + j, d[j]) != d + j)
+				return false;
+		}
+	}
+	int64_t sum = 0;
+	for (int64_t r = 0; r < n; ++r)
+		sum += net[pid[r]];
+	return sum == 0;
+}
+
 // Grid stencil: the positive offsets are 1, nx and nx ny (one, two or three
 // of them) and every row r = i + nx (j + ny k) holds exactly its neighbours
 // inside the nx x ny x nz grid, in column order.  Rows fall in at most 64
@@ -869,6 +889,7 @@ FS_API int fs_csr_create(fs_ctx h, int64_t nrows, int64_t ncols, int64_t nnz,
 			}
 			A->nsym = (int)sofs.size();
 			A->sym_ld = sym_ld;
+			A->sym_paired = paired(nrows, ptab, plen, npat, pid);
 			int dims[3];
 			if (grid_dims(nrows, sofs, pid, ptab, plen, dims)) {
 				A->grid_nx = dims[0];

@@ -443,7 +443,8 @@ FS_API int fs_krylov_mixed_stats(fs_solver s, int *outer, int *inner_iters);
 /* ------------------------------------------------------------ adjoint --- */
 /* No counterpart in the reference (it has no adjoint).  For a loss L(x) of
  * x = A^-1 b:  A^T lambda = dL/dx (fs_krylov_apply_transpose: the bound
- * solver on the transposed operator, a CSC view of A built once per pattern),
+ * solver on the transposed operator, a CSC view of A built once per pattern,
+ * or on A itself when pattern and values are known to be symmetric),
  * dL/db = lambda, dL/dA_ij = -lambda_i x_j (fs_csr_value_grad), and for the
  * finite-volume diffusion operator assembled from face coefficients
  * (fs_fv_assemble, same face layout and row order as the seeded generators)

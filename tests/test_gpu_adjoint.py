@@ -284,3 +284,68 @@ def test_heat_backward_euler_adjoint_64(ctx):
     for i in coords:
         fd = _heat_fd(ctx, sm, sp, c, u0, target, nsteps, int(i), dt)
         assert abs(g[i] - fd) <= FD_RTOL * abs(fd), (int(i), g[i], fd)
+
+
+# ------------------------------------- transposes of one-sided patterns ---
+
+def _csr(M, name):
+    M = M.tocsr()
+    M.sort_indices()
+    return P.CSR(M.shape[0], M.shape[1], M.indptr.astype(np.int64), M.indices.astype(np.int32),
+                 M.data.astype(np.float64), name)
+
+
+def _one_sided(kind, n=24):
+    """Operators of few offsets, each diagonally dominant by rows and columns:
+    (matrix, whether it equals its transpose)."""
+    import scipy.sparse as sp
+    N = n * n
+    one = lambda d, v=-1.0: sp.diags([np.full(N - abs(d), v)], [d], shape=(N, N))
+    I = sp.identity(N)
+    if kind == "upper-bidiagonal":
+        return _csr(4 * I + one(1), kind), False
+    if kind == "upwind":          # couplings +1 and +n alone
+        return _csr(4 * I + one(1) + one(n), kind), False
+    if kind == "lower-bidiagonal":
+        return _csr(4 * I + one(-1), kind), False
+    if kind == "missing-partner":  # a 2-D stencil without one lower entry
+        A = P.diffusion(2, n, seed=3).to_scipy().tolil()
+        A[5 * n, 4 * n] = 0
+        A = A.tocsr()
+        A.eliminate_zeros()
+        return _csr(A, kind), False
+    if kind == "missing-pair":     # and without its partner
+        A = P.diffusion(2, n, seed=3).to_scipy().tolil()
+        A[5 * n, 4 * n] = A[4 * n, 5 * n] = 0
+        A = A.tocsr()
+        A.eliminate_zeros()
+        return _csr(A, kind), True
+    if kind == "swapped-pairs":    # as many upper as lower entries, not the same
+        A = (8 * I + one(1) + one(-1) + one(n) + one(-n)).tolil()
+        A[5 * n, 4 * n] = 0
+        A[7 * n, 8 * n] = 0
+        A = A.tocsr()
+        A.eliminate_zeros()
+        return _csr(A, kind), False
+    return _csr(10 * I + sum(one(s * d) for s in (1, -1) for d in (1, n - 1, n, n + 1)), kind), True
+
+
+@pytest.mark.parametrize("kind", ["upper-bidiagonal", "lower-bidiagonal", "upwind", "missing-partner",
+                                  "missing-pair", "swapped-pairs", "nine-point"])
+def test_transpose_solve_of_few_offset_patterns(ctx, kind):
+    """A^T x = b for patterns that hold an upper entry without a lower
+    partner: stopped at 1e-10, the residual of A^T is at most twice that (the
+    recurrence's estimate against the true one); the forward solve's bits only
+    where A is its own transpose."""
+    A, own = _one_sided(kind)
+    S = A.to_scipy()
+    assert own == ((S != S.T).nnz == 0)
+    b = P.uniform(5, A.nrows)
+    vb, vf, vt = fs.Vector(ctx, b), fs.Vector(ctx, A.nrows), fs.Vector(ctx, A.nrows)
+    slv = fs.bicgstab.solver(fs.bicgstab.settings(maxiter=2000, rtol=1e-10))(fs.CSR(ctx, A), fs.op.jacobi)
+    assert slv(vb, vf).status == slv.apply_transpose(vb, vt).status == "converged_rtol"
+    xf, xt = vf.numpy(), vt.numpy()
+    assert np.linalg.norm(b - S @ xf) <= 2e-10 * np.linalg.norm(b)
+    assert np.linalg.norm(b - S.T @ xt) <= 2e-10 * np.linalg.norm(b)
+    if own:
+        assert np.linalg.norm(xf - xt) <= 1e-8 * np.linalg.norm(xf)
