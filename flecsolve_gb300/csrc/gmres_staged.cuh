@@ -514,7 +514,7 @@ k_gm_staged(OrthoArgs<T> a, const __grid_constant__ BasisMaps maps) {
 			}
 			__syncthreads();
 			if (warp == 0) {
-				const double r = k > 0 ? sqrt(fmax(s[k] - dots[0], 0.0)) : 1.0;
+				const double r = k > 0 ? gm_norm(s[k] - dots[0]) : 1.0;
 				const double rinv = r != 0.0 ? 1.0 / r : 1.0;
 				if (lane == 0) {
 					dots[0] = r;
@@ -583,7 +583,7 @@ k_gm_staged(OrthoArgs<T> a, const __grid_constant__ BasisMaps maps) {
 					double s2 = 0.0;
 					for (int j = 0; j < kp1; ++j)
 						s2 += folded[j] * folded[j];
-					const double vn2 = sqrt(fmax(folded[kp1] - s2, 0.0));
+					const double vn2 = gm_norm(folded[kp1] - s2);
 					g->H[kp1 + ldh * k] = vn2;
 					g->vnorm = vn2;
 				}

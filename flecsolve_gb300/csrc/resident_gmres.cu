@@ -509,7 +509,7 @@ k_gm_resident(ResGm<T> a) {
 						hs[lane] = (T)q[0];
 						ht[lane] = (T)q[1];
 					}
-					const double r = k > 0 ? sqrt(fmax(alpha - ss, 0.0)) : 1.0;
+					const double r = k > 0 ? gm_norm(alpha - ss) : 1.0;
 					const double rinv = r != 0.0 ? 1.0 / r : 1.0;
 					if (lane == 0) {
 						st.r = r;

@@ -67,6 +67,11 @@ struct GmState {
 	int pad_;
 };
 
+// the norm of a vector from the difference of two sums of squares: 0 where
+// rounding left it negative; a NaN stays one, so that the estimate formed from
+// it is not finite either
+__device__ __forceinline__ double gm_norm(double d) { return d > 0.0 ? sqrt(d) : d == d ? 0.0 : d; }
+
 struct Solver;
 struct ResSlots;
 

@@ -267,3 +267,31 @@ def test_resident_gmres_estimate_is_the_true_residual(ctx, method, u, shape, dim
             first = h, x
         else:
             assert np.array_equal(h, first[0]) and np.array_equal(x, first[1])
+
+
+# ---------------------------------------------------- values not finite ---
+
+GM = dict(max_krylov_dim=30, restart=True)
+
+
+@pytest.mark.parametrize("coding", ["grid", "patterns"])
+@pytest.mark.parametrize("method,kw", [("gmres", dict(GM, ortho=o, pre_side=p))
+                                       for o in ("auto", "mgs", "cgs2", "dcgs2") for p in ("right", "left")] +
+                         [("mixed_gmres", dict(GM, ortho=o)) for o in ("auto", "cgs2")] +
+                         [("bicgstab", dict()), ("mixed_bicgstab", dict())])
+def test_gmres_and_bicgstab_report_non_finite(ctx, method, kw, coding):
+    """A NaN or an infinity in the matrix, the right-hand side or the guess
+    ends every solver with the non-finite status (5), never as converged."""
+    A = _grid(40, 36, 1, 2, seed=1, asym=0.2)
+    b, x0 = P.uniform(4, A.nrows), P.uniform(9, A.nrows)
+    at = int(np.flatnonzero(A.col == 700)[1])
+    for bad in (np.nan, np.inf):
+        v = A.val.copy()
+        v[at] = bad
+        B = P.CSR(A.nrows, A.ncols, A.rowptr, A.col, v)
+        c, y0 = b.copy(), x0.copy()
+        c[7] = y0[9] = bad
+        for M, rhs, guess in ((B, b, None), (B, b, x0), (A, c, None), (A, c, x0), (A, b, y0)):
+            with pytest.raises(FsError) as e:
+                _solve(ctx, M, rhs, method, coding, x0=guess, maxiter=90, rtol=1e-9, **kw)
+            assert e.value.status == 5
