@@ -522,14 +522,14 @@ int gen_gmres(Gen &g, Vec *b, Vec *x, fs_solve_info *info) {
 		FS_TRY(g.copy(v, V[k + 1]));
 		for (int i = 0; i < k; ++i)
 			ls.apply_givens(i, k);
-		if (v_norm != 0.0) {
-			ls.compute_givens(k);
-			ls.apply_givens(k, k);
-			ls.h(k + 1, k) = 0.0;
-			const double xx = ls.dw[k], c = ls.cs[k], sn = ls.sn[k];
-			ls.dw[k] = c * xx;
-			ls.dw[k + 1] = -sn * xx;
-		}
+		// (a column without a remainder takes the identity, where the
+		// reference leaves the rotation and dw[k + 1] of the cycle before)
+		ls.compute_givens(k);
+		ls.apply_givens(k, k);
+		ls.h(k + 1, k) = 0.0;
+		const double xx = ls.dw[k], c = ls.cs[k], sn = ls.sn[k];
+		ls.dw[k] = c * xx;
+		ls.dw[k + 1] = -sn * xx;
 		v_norm = std::fabs(ls.dw[k + 1]);
 		++k;
 		int stop;

@@ -149,17 +149,16 @@ __device__ void compute_givens(GmState *g, int k) {
 __device__ void finish_step(GmState *g, KState *st, double *hist) {
 	const int k = g->k;
 	const int ld = g->ld;
-	const double vnorm = g->vnorm;
 	for (int i = 0; i < k; i++)
 		apply_givens(g, i, k);
-	if (vnorm != 0.0) {
-		compute_givens(g, k);
-		apply_givens(g, k, k);
-		g->H[k + 1 + ld * k] = 0.0;
-		double x = g->dw[k], c = g->cs[k], s = g->sn[k];
-		g->dw[k] = c * x;
-		g->dw[k + 1] = -s * x;
-	}
+	// (a column without a remainder takes the identity, where the reference
+	// leaves the rotation and dw[k + 1] of the cycle before)
+	compute_givens(g, k);
+	apply_givens(g, k, k);
+	g->H[k + 1 + ld * k] = 0.0;
+	const double x = g->dw[k], c = g->cs[k], s = g->sn[k];
+	g->dw[k] = c * x;
+	g->dw[k + 1] = -s * x;
 	const double res = fabs(g->dw[k + 1]);
 	g->k = k + 1;
 	const int it = st->iter + 1;
@@ -211,34 +210,30 @@ __device__ void finish_step_warp(GmState *g, KState *st, double *hist, double *c
 		x = __shfl_sync(0xffffffffu, v, 1);
 	}
 	if (lane == 0) {
-		const double vnorm = g->vnorm;
-		if (vnorm != 0.0) {
-			const double f = x, gg = col[k + 1];
-			double c, s;
-			if (gg == 0.0) {
-				c = 1.0;
-				s = 0.0;
-			}
-			else if (f == 0.0) {
-				c = 0.0;
-				s = (gg < 0.0) ? -1.0 : 1.0;
-			}
-			else {
-				double r = sqrt(f * f + gg * gg);
-				r = 1.0 / r;
-				c = fabs(f) * r;
-				s = copysign(gg * r, f);
-			}
-			g->cs[k] = c;
-			g->sn[k] = s;
-			col[k] = c * f + s * gg;
-			col[k + 1] = 0.0;
-			const double w = g->dw[k];
-			g->dw[k] = c * w;
-			g->dw[k + 1] = -s * w;
+		// (a column without a remainder: the identity)
+		const double f = x, gg = col[k + 1];
+		double c, s;
+		if (gg == 0.0) {
+			c = 1.0;
+			s = 0.0;
 		}
-		else
-			col[k] = x;
+		else if (f == 0.0) {
+			c = 0.0;
+			s = (gg < 0.0) ? -1.0 : 1.0;
+		}
+		else {
+			double r = sqrt(f * f + gg * gg);
+			r = 1.0 / r;
+			c = fabs(f) * r;
+			s = copysign(gg * r, f);
+		}
+		g->cs[k] = c;
+		g->sn[k] = s;
+		col[k] = c * f + s * gg;
+		col[k + 1] = 0.0;
+		const double w = g->dw[k];
+		g->dw[k] = c * w;
+		g->dw[k + 1] = -s * w;
 		const double res = fabs(g->dw[k + 1]);
 		g->k = k + 1;
 		const int it = st->iter + 1;

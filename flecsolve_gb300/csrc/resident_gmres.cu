@@ -170,24 +170,28 @@ __device__ void rg_finish_column(RgSmall &g, const RgStep &st, int c, double *hi
 	if (lane == 0) {
 		const double gg = st.r;
 		col[c] = x;
-		if (gg != 0.0) {
-			double cc, s;
-			if (x == 0.0) {
-				cc = 0.0;
-				s = gg < 0.0 ? -1.0 : 1.0;
-			}
-			else {
-				const double q = 1.0 / sqrt(x * x + gg * gg);
-				cc = fabs(x) * q;
-				s = copysign(gg * q, x);
-			}
-			g.cs[c] = cc;
-			g.sn[c] = s;
-			col[c] = cc * x + s * gg;
-			const double w = g.dw[c];
-			g.dw[c] = cc * w;
-			g.dw[c + 1] = -s * w;
+		// a column without a remainder takes the identity: its estimate
+		// is 0 and not what the cycle before left in dw[c + 1]
+		double cc, s;
+		if (gg == 0.0) {
+			cc = 1.0;
+			s = 0.0;
 		}
+		else if (x == 0.0) {
+			cc = 0.0;
+			s = gg < 0.0 ? -1.0 : 1.0;
+		}
+		else {
+			const double q = 1.0 / sqrt(x * x + gg * gg);
+			cc = fabs(x) * q;
+			s = copysign(gg * q, x);
+		}
+		g.cs[c] = cc;
+		g.sn[c] = s;
+		col[c] = cc * x + s * gg;
+		const double w = g.dw[c];
+		g.dw[c] = cc * w;
+		g.dw[c + 1] = -s * w;
 		const double res = fabs(g.dw[c + 1]);
 		g.k = c + 1;
 		g.it += 1;

@@ -295,3 +295,35 @@ def test_gmres_and_bicgstab_report_non_finite(ctx, method, kw, coding):
             with pytest.raises(FsError) as e:
                 _solve(ctx, M, rhs, method, coding, x0=guess, maxiter=90, rtol=1e-9, **kw)
             assert e.value.status == 5
+
+
+# ------------------------------------ an exact breakdown after a restart ---
+
+def _breakdown(n):
+    """GMRES(1) on this matrix leaves an exact eigenvector after its first
+    cycle, every product and sum of both cycles being exact: |H(1, 0)| = 0 in
+    the second.  A 1-D stencil that couples row 0 to row 1 alone."""
+    A = _grid(n, 1, 1, 1, seed=1, asym=0.5)
+    rows = np.repeat(np.arange(n), np.diff(A.rowptr))
+    v = np.where(rows == A.col, 2.0, 0.0)
+    v[0] = 1.0
+    v[1] = -1.0
+    return P.CSR(n, n, A.rowptr, A.col, v)
+
+
+@pytest.mark.parametrize("n", [16, 256, 4096])
+@pytest.mark.parametrize("route", ["grid", "patterns", "mgs", "cgs2", "shell"])
+def test_gmres_exact_breakdown_in_the_second_cycle(ctx, n, route):
+    """The estimate of a column without a rotation is 0, not the one that the
+    cycle before left: converged after two iterations, on every route."""
+    A = _breakdown(n)
+    b = np.ones(n)
+    dA, vb, vx = fs.CSR(ctx, A), fs.Vector(ctx, b), fs.Vector(ctx, n)
+    dA.index_coding("grid" if route == "grid" else "patterns")
+    op = fs.op.make_shell(ctx, lambda x, y: dA.apply(x, y), n) if route == "shell" else fs.op.ref(dA)
+    ortho = dict(ortho=route) if route in ("mgs", "cgs2") else dict(ortho="dcgs2")
+    s = fs.gmres.settings(maxiter=10, rtol=1e-12, use_zero_guess=True, max_krylov_dim=1, restart=True, **ortho)
+    slv = fs.gmres.solver(s, fs.gmres.make_work(vb))(op, fs.op.I)
+    info = slv(vb, vx)
+    assert (info.status, info.iters, info.restarts) == ("converged_rtol", 2, 1)
+    assert np.array_equal(A.to_scipy() @ vx.numpy(), b)
