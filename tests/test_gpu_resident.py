@@ -327,3 +327,62 @@ def test_gmres_exact_breakdown_in_the_second_cycle(ctx, n, route):
     info = slv(vb, vx)
     assert (info.status, info.iters, info.restarts) == ("converged_rtol", 2, 1)
     assert np.array_equal(A.to_scipy() @ vx.numpy(), b)
+
+
+# ------------------------------- BiCGSTAB's breakdowns and its restart ---
+
+# 4 x 4 tridiagonal blocks and right-hand sides on which the first iteration is
+# exact (dyadic numbers): (a, b, what it meets)
+BI_BLOCKS = {
+    # skew: r~'A r = 0
+    "alpha": ([[0, 1, 0, 0], [-1, 0, 0, 0], [0, 0, 0, 1], [0, 0, -1, 0]], [1, 1, 1, 1]),
+    # t's = 0, t't = 3: omega = 0
+    "omega": ([[-.5, 0, 0, 0], [0, 1.5, 0, 0], [0, 0, 1.5, 0], [0, 0, 0, 1.5]], [1, 1, 1, 1]),
+    # r~'res = 0 after one iteration: restart from the true residual
+    "restart": ([[-2, -1, 0, 0], [2, -1, 0, 0], [0, 1, 1, 1], [0, 0, -1, 0]], [1, -1, 1, -1]),
+    "restart-2": ([[2, 0, 0, 0], [-3, -.5, 1, 0], [0, 3, 0, 0], [0, 0, 0, 1]], [-1, 2, 2, 2]),
+}
+
+
+def _blocks(kind, copies):
+    a, b = BI_BLOCKS[kind]
+    n = 4 * copies
+    A = _grid(n, 1, 1, 1, seed=1, asym=0.5)
+    rows = np.repeat(np.arange(n), np.diff(A.rowptr))
+    same = rows // 4 == A.col // 4
+    v = np.where(same, np.array(a)[rows % 4, A.col % 4], 0.0)
+    return P.CSR(n, n, A.rowptr, A.col, v), np.tile(np.array(b, np.float64), copies)
+
+
+@pytest.mark.parametrize("copies", [4, 64, 1024])
+@pytest.mark.parametrize("kind", sorted(BI_BLOCKS))
+def test_resident_bicgstab_breakdowns_and_restart(ctx, kind, copies):
+    """r~'A P r = 0, omega = 0 and the restart at r~'res = 0, each met exactly:
+    the error of the first, else the phase kernels' status, counts, restarts and solution, after every
+    number of iterations up to 5, from a zero and a given guess, and the
+    stopping test met by the true residual where a solve converges."""
+    A, b = _blocks(kind, copies)
+    M = A.to_scipy()
+    x0 = np.ones(A.nrows)
+    for guess, rhs in ((None, b), (x0, b + M @ x0)):
+        for maxiter in (1, 2, 3, 4, 5, 200):
+            kw = dict(maxiter=maxiter, rtol=1e-8, x0=guess, jacobi=False)
+            if kind == "alpha":
+                for coding in ("grid", "patterns"):
+                    with pytest.raises(FsError, match="alpha = 0"):
+                        _solve(ctx, A, rhs, "bicgstab", coding, **kw)
+                continue
+            one, x1, h1, l1 = _solve(ctx, A, rhs, "bicgstab", "grid", **kw)
+            ref, x2, h2, l2 = _solve(ctx, A, rhs, "bicgstab", "patterns", **kw)
+            assert l1 < l2
+            assert one.status == ref.status
+            if maxiter <= 5:
+                assert (one.iters, one.restarts, h1.size) == (ref.iters, ref.restarts, h2.size)
+                assert np.allclose(h1, h2, rtol=1e-9, atol=1e-12 * np.linalg.norm(b))
+                assert np.allclose(x1, x2, rtol=1e-9, atol=1e-9)
+            if kind == "omega":
+                assert (one.status, one.iters, h1.size) == ("diverged_breakdown", 1, 1)
+            elif maxiter > 1:
+                assert one.restarts >= 1
+            if one.success():
+                assert np.linalg.norm(rhs - M @ x1) <= 2e-8 * np.linalg.norm(rhs)
