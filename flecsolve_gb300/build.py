@@ -130,6 +130,17 @@ def build_template_test(force: bool = False):
     return out
 
 
+def build_math_test(force: bool = False) -> Path:
+    """The resident kernels' scalar arithmetic on arrays of operands
+    (tests/cpp/test_resident_math.cu), a shared object of its own."""
+    BUILD.mkdir(exist_ok=True)
+    out = BUILD / "test_resident_math.so"
+    src = ROOT / "tests" / "cpp" / "test_resident_math.cu"
+    if force or _stale(out, [src, *CSRC.glob("*.cuh"), *INCLUDE.glob("*.h")]):
+        _run([_nvcc(), *ARCH, *NVCC_FLAGS, "-shared", "-o", str(out), str(src), "-lcudart"])
+    return out
+
+
 def build_oracle() -> None:
     oracle = str(ROOT / "oracle")
     ref = os.environ.get("FLECSOLVE_REF")
@@ -144,6 +155,7 @@ def build_all(force: bool = False, verbose: bool = False) -> None:
     build_gpu(force, verbose)
     build_cpp_tests(force)
     build_template_test(force)
+    build_math_test(force)
 
 
 if __name__ == "__main__":

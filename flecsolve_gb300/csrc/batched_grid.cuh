@@ -75,24 +75,6 @@ __device__ __forceinline__ void bg_rows_do(int cnt, F &&f) {
 	}
 }
 
-// a / b rounded to FP32 (to half a unit and a 2^-40th): the leading parts'
-// quotient and its residual, in FP32 on the mantissas; 20 short operations
-// where the FP64 division holds the one warp that everything waits for 561
-// cycles
-__device__ __forceinline__ float bg_quotient(double a, double b) {
-	const long long ua = __double_as_longlong(a), ub = __double_as_longlong(b);
-	const int ea = (int)(ua >> 52) & 0x7ff, eb = (int)(ub >> 52) & 0x7ff, e = ea - eb;
-	if (ea == 0 || eb == 0 || ea == 0x7ff || eb == 0x7ff || e < -120 || e > 120)
-		return (float)(a / b);
-	const float ah = __int_as_float(0x3f800000 | ((int)(ua >> 29) & 0x7fffff));
-	const float bh = __int_as_float(0x3f800000 | ((int)(ub >> 29) & 0x7fffff));
-	const float al = (float)((int)ua & 0x1fffffff) * 0x1p-52f, bl = (float)((int)ub & 0x1fffffff) * 0x1p-52f;
-	const float y = __frcp_rn(bh), q = ah * y;
-	const float r = fmaf(-q, bh, ah) + fmaf(-q, bl, al);
-	const float v = fmaf(r, y, q) * __int_as_float((e + 127) << 23);
-	return (ua ^ ub) < 0 ? -v : v;
-}
-
 // floats of dynamic shared memory: p with two halos, the upper diagonals (the
 // outer one with a halo of lower partners, the inner one with one row), the
 // diagonal, D^-1, z of the halo rows.  The head's doubles (p with two halos,
@@ -483,7 +465,7 @@ k_batch_grid(BatchArgs a) {
 				const double q = team_sum(fq);
 				if (tid == 0) {
 					sh.rho = sh.rz;
-					sh.af = bg_quotient(sh.rz, q);
+					sh.af = res_quotient32(sh.rz, q);
 				}
 				__syncthreads();
 				const float af = sh.af;
@@ -513,7 +495,7 @@ k_batch_grid(BatchArgs a) {
 				}
 				if (tid == 32) {
 					sh.rz = t;
-					sh.bf = bg_quotient(t, sh.rho);
+					sh.bf = res_quotient32(t, sh.rho);
 				}
 				__syncthreads();
 				float bf = sh.bf;

@@ -324,19 +324,6 @@ __device__ void back_solve_warp(GmState *g) {
 		back_solve_rows<1>(g);
 }
 
-// (double)v of a normal number or zero in integer operations: the conversion
-// takes the FP64 pipe as long as an FMA does
-__device__ __forceinline__ double widen(float v) {
-	const unsigned b = __float_as_uint(v), a = b & 0x7fffffffu;
-	return __hiloint2double((int)((a ? (a >> 3) + 0x38000000u : 0u) | (b & 0x80000000u)), (int)(a << 29));
-}
-__device__ __forceinline__ bool widens(float v) {
-	const unsigned a = __float_as_uint(v) & 0x7fffffffu;
-	return a - 1u >= 0x7fffffu && a < 0x7f800000u;  // not subnormal, finite
-}
-__device__ __forceinline__ double widen(double v) { return v; }
-__device__ __forceinline__ bool widens(double) { return true; }
-
 // z + sum_u c[u] v[u] with conversions (its own function: in line, the compiler
 // converts on both sides of the branch that leads here)
 template<int N, class T>

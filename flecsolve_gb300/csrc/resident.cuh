@@ -51,7 +51,8 @@ constexpr int kResPolls = 1 << 22;
 // below 2^-30 of the unit in the last place of the group's largest value, a
 // warp's sum is rounded to an eighth of that unit and a CTA's to the unit, so
 // the result is at least as accurate as the tree's, and it does not depend on
-// the order of the values.
+// the order of the values.  FP32 values lose bits below 2^-29 of the largest
+// one's FP32 unit (a double's last bit).
 
 // a group's sum q 2^(e - 1075 - F), F = 3 for a warp, 0 for a CTA; e = 0x7ff:
 // some value was not finite, q the union of 1 (+inf), 2 (-inf) and 4 (NaN)
@@ -494,9 +495,9 @@ __device__ __forceinline__ double res_quotient(double a, double b, double y) {
 	return safe ? r : a / b;
 }
 
-// a / b to half a unit in the last place and 2^-37 of one: b's reciprocal from
-// the FP32 one of its leading bits and one Newton step (2^-45), the quotient's
-// residual as above.  Five dependent FP64 operations on the path of a sum that
+// a / b to half a unit in the last place and 2^-36 of one: b's reciprocal from
+// the FP32 one of its leading bits (1.5 x 2^-23) and one Newton step (2^-44.8),
+// the quotient's residual as above.  Five dependent FP64 operations on the path of a sum that
 // everything waits for; the division takes ten.
 __device__ __forceinline__ double res_divide(double a, double b) {
 	const int ea = res_exponent(a), eb = res_exponent(b), hi = __double2hiint(b);
@@ -512,6 +513,38 @@ __device__ __forceinline__ double res_divide(double a, double b) {
 	const double q = a * y;
 	return fma(fma(-q, b, a), y, q);
 }
+
+// a / b rounded to FP32, to half a unit and 2^-40 of the value: the quotient of
+// the leading parts, corrected by the residual of both parts (Dekker 1971, "A
+// floating-point technique for extending the available precision"), in FP32 on
+// the mantissas; 20 short operations where the FP64 division holds the one warp
+// that everything waits for 561 cycles
+__device__ __forceinline__ float res_quotient32(double a, double b) {
+	const long long ua = __double_as_longlong(a), ub = __double_as_longlong(b);
+	const int ea = (int)(ua >> 52) & 0x7ff, eb = (int)(ub >> 52) & 0x7ff, e = ea - eb;
+	if (ea == 0 || eb == 0 || ea == 0x7ff || eb == 0x7ff || e < -120 || e > 120)
+		return (float)(a / b);
+	const float ah = __int_as_float(0x3f800000 | ((int)(ua >> 29) & 0x7fffff));
+	const float bh = __int_as_float(0x3f800000 | ((int)(ub >> 29) & 0x7fffff));
+	const float al = (float)((int)ua & 0x1fffffff) * 0x1p-52f, bl = (float)((int)ub & 0x1fffffff) * 0x1p-52f;
+	const float y = __frcp_rn(bh), q = ah * y;
+	const float r = fmaf(-q, bh, ah) + fmaf(-q, bl, al);
+	const float v = fmaf(r, y, q) * __int_as_float((e + 127) << 23);
+	return (ua ^ ub) < 0 ? -v : v;
+}
+
+// (double)v of a normal number or zero in integer operations: the conversion
+// takes the FP64 pipe as long as an FMA does
+__device__ __forceinline__ double widen(float v) {
+	const unsigned b = __float_as_uint(v), a = b & 0x7fffffffu;
+	return __hiloint2double((int)((a ? (a >> 3) + 0x38000000u : 0u) | (b & 0x80000000u)), (int)(a << 29));
+}
+__device__ __forceinline__ bool widens(float v) {
+	const unsigned a = __float_as_uint(v) & 0x7fffffffu;
+	return a - 1u >= 0x7fffffu && a < 0x7f800000u;  // not subnormal, finite
+}
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ bool widens(double) { return true; }
 
 // the payload of a packet that had not arrived at the first look (its own
 // function: inlined, the loops of a row's neighbours cost the caller spills)
