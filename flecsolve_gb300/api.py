@@ -681,6 +681,11 @@ class BoundSolver:
         check(lib().fs_krylov_history(self.h, out.ctypes.data_as(_lib._dp), C.byref(m)), self.ctx.h)
         return out[: m.value]
 
+    def wait_limit(self, reads: int) -> None:
+        """Looks at another CTA's message after which a solve in one
+        cooperative launch gives up with an error (0: the default)."""
+        check(lib().fs_krylov_wait_limit(self.h, int(reads)), self.ctx.h, "fs_krylov_wait_limit")
+
     def mixed_stats(self):
         o, i = C.c_int(), C.c_int()
         check(lib().fs_krylov_mixed_stats(self.h, C.byref(o), C.byref(i)), self.ctx.h)

@@ -2444,6 +2444,16 @@ FS_API int fs_krylov_history(fs_solver h, double *hist, int64_t *n) {
 	return FS_OK;
 }
 
+FS_API int fs_krylov_wait_limit(fs_solver h, int reads) {
+	Solver *s = reinterpret_cast<Solver *>(h);
+	if (!ok_slv(s))
+		return FS_ERR_BAD_HANDLE;
+	if (reads < 0)
+		return set_err(s->ctx, FS_ERR_INVALID_ARG, "fs_krylov_wait_limit: negative limit");
+	s->res_polls = reads;
+	return FS_OK;
+}
+
 FS_API int fs_krylov_mixed_stats(fs_solver h, int *outer, int *inner) {
 	Solver *s = reinterpret_cast<Solver *>(h);
 	if (!ok_slv(s))

@@ -34,6 +34,7 @@ struct ResCg {
 	int maxiter, hist_cap, zero_guess;
 	int rows;                 // rows per CTA
 	int smem;                 // dynamic shared memory, bytes
+	int polls;
 };
 
 // PKT: the slice's p fits in shared memory and the other slices read it as
@@ -52,7 +53,7 @@ k_cg_resident(ResCg a) {
 	};
 	__shared__ Scalars z;
 	ResTeam tm;
-	tm.init(a.slots, &sh, a.err);
+	tm.init(a.slots, &sh, a.err, a.polls);
 	const int tid = threadIdx.x, nt = blockDim.x;
 	const int lo = (int)min((int64_t)blockIdx.x * a.rows, (int64_t)a.A.n);
 	const int cnt = (int)min((int64_t)a.rows, (int64_t)a.A.n - lo);
@@ -343,6 +344,7 @@ int cg_apply_resident(Solver *s, Vec *b, Vec *x, fs_solve_info *info, int *taken
 	a.hist = s->hist;
 	a.slots = s->res_slots;
 	a.err = ctx->dev_err;
+	a.polls = res_polls(s);
 	a.rtol = (double)s->set.base.rtol;
 	a.maxiter = s->set.base.maxiter;
 	a.hist_cap = s->hist_cap;
@@ -352,7 +354,7 @@ int cg_apply_resident(Solver *s, Vec *b, Vec *x, fs_solve_info *info, int *taken
 	FS_TRY(res_launch(ctx, kern, sh, a, "resident cg", taken));
 	if (!*taken)
 		return FS_OK;
-	FS_TRY(read_state(s));
+	FS_TRY(res_read_state(s));
 	const KState &h = *s->hst;
 	s->hhist_count = std::min<int64_t>(h.iter, s->hist_cap);
 	memset(info, 0, sizeof(*info));
@@ -370,6 +372,26 @@ int cg_apply_resident(Solver *s, Vec *b, Vec *x, fs_solve_info *info, int *taken
 	return FS_OK;
 }
 
+// no slot or packet carries the epoch a first launch starts from
+static cudaError_t first_epoch(Solver *s, ResSlots *p) {
+	return cudaMemsetAsync(&p->epoch, 1, 1, s->ctx->stream);
+}
+
+int res_read_state(Solver *s) {
+	const int st = read_state(s);
+	if (st != FS_OK) {
+		cudaStream_t q = s->ctx->stream;
+		cudaMemsetAsync(s->res_slots, 0, sizeof(ResSlots), q);
+		first_epoch(s, s->res_slots);
+		if (s->res_pk)
+			cudaMemsetAsync(s->res_pk, 0, (size_t)s->n * sizeof(ulonglong2), q);
+		if (s->res_vals)
+			cudaMemsetAsync(s->res_vals, 0, s->res_vals_len, q);
+		cudaGetLastError();
+	}
+	return st;
+}
+
 bool res_memory(Solver *s, bool packets) {
 	// one buffer of zeroes; false (and no error left) when there is no room
 	auto get = [&](size_t bytes) -> void * {
@@ -382,9 +404,8 @@ bool res_memory(Solver *s, bool packets) {
 		return cudaMemsetAsync(p, 0, bytes, s->ctx->stream) == cudaSuccess ? p : nullptr;
 	};
 	if (!s->res_slots) {
-		// no slot or packet carries the epoch a first launch starts from
 		auto *p = (ResSlots *)get(sizeof(ResSlots));
-		if (!p || cudaMemsetAsync(&p->epoch, 1, 1, s->ctx->stream) != cudaSuccess)
+		if (!p || first_epoch(s, p) != cudaSuccess)
 			return false;
 		s->res_slots = p;
 	}

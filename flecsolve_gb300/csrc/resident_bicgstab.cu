@@ -29,7 +29,7 @@ struct ResBi {
 	unsigned *err;
 	double rtol;
 	int maxiter, hist_cap, zero_guess;
-	int rows, smem;
+	int rows, smem, polls;
 };
 
 template<int K, bool GEN>
@@ -47,7 +47,7 @@ k_bi_resident(ResBi a) {
 	__shared__ Scalars z;
 	__shared__ ResRows<double, K, GEN> A;
 	ResTeam tm;
-	tm.init(a.slots, &sh, a.err);
+	tm.init(a.slots, &sh, a.err, a.polls);
 	const int tid = threadIdx.x, nt = blockDim.x;
 	const int lo = (int)min((int64_t)blockIdx.x * a.rows, (int64_t)a.A.n);
 	const int cnt = (int)min((int64_t)a.rows, (int64_t)a.A.n - lo);
@@ -440,6 +440,7 @@ int bicgstab_apply_resident(Solver *s, Vec *b, Vec *x, int *taken) {
 	a.hist = s->hist;
 	a.slots = s->res_slots;
 	a.err = ctx->dev_err;
+	a.polls = res_polls(s);
 	a.rtol = (double)s->set.base.rtol;
 	a.maxiter = s->set.base.maxiter;
 	a.hist_cap = s->hist_cap;
@@ -449,7 +450,7 @@ int bicgstab_apply_resident(Solver *s, Vec *b, Vec *x, int *taken) {
 	FS_TRY(res_launch(ctx, kern, sh, a, "resident bicgstab", taken));
 	if (!*taken)
 		return FS_OK;
-	return read_state(s);
+	return res_read_state(s);
 }
 
 }  // namespace fsg

@@ -52,7 +52,7 @@ struct ResGm {
 	double *hist;
 	double rtol;
 	int maxiter, hist_cap, zero_guess, right, m, mixed;
-	int rows, smem;
+	int rows, smem, polls;
 };
 
 // rows a thread takes at a time in the basis passes: 16 bytes of FP32 rows
@@ -230,7 +230,7 @@ k_gm_resident(ResGm<T> a) {
 	__shared__ T *col[kGmDelayedCols];    // the slice's rows of each column
 	__shared__ T hs[kGmDelayedCols], ht[kGmDelayedCols];
 	ResTeam tm;
-	tm.init(a.slots, &sh, a.err);
+	tm.init(a.slots, &sh, a.err, a.polls);
 	const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5;
 	const int nwk = (nt >> 5) - 1, ntk = nwk * 32;  // workers; the last warp keeps the Hessenberg
 	const bool worker = wid < nwk;
@@ -485,7 +485,7 @@ k_gm_resident(ResGm<T> a) {
 					double q[2] = {0.0, 0.0};
 					bool here = false;
 					res_hold(clock64());
-					for (int it = 0; !here && it < kResPolls; ++it) {
+					for (int it = 0; !here && it < sh.polls; ++it) {
 						ulonglong2 m[2];
 #pragma unroll
 						for (int i = 0; i < 2; ++i)
@@ -754,6 +754,7 @@ int gmres_apply_resident(Solver *s, Vec *b, Vec *x, int m, bool mixed, int *take
 		s->bufs.push_back(p);
 		FS_CUDA_TRY(ctx, cudaMemsetAsync(p, 0, sizeof(RgSlots), ctx->stream));
 		s->res_vals = p;
+		s->res_vals_len = sizeof(RgSlots);
 	}
 	FS_TRY(solver_hist(s, std::max(1, s->set.base.maxiter)));
 	if constexpr (sizeof(T) == 8)
@@ -770,6 +771,7 @@ int gmres_apply_resident(Solver *s, Vec *b, Vec *x, int m, bool mixed, int *take
 	a.vals = (RgSlots *)s->res_vals;
 	a.slots = s->res_slots;
 	a.err = ctx->dev_err;
+	a.polls = res_polls(s);
 	a.st = s->st;
 	a.hist = s->hist;
 	a.rtol = (double)s->set.base.rtol;
@@ -784,7 +786,7 @@ int gmres_apply_resident(Solver *s, Vec *b, Vec *x, int m, bool mixed, int *take
 	FS_TRY(res_launch(ctx, kern, sh, a, "resident gmres", taken));
 	if (!*taken)
 		return FS_OK;
-	return read_state(s);
+	return res_read_state(s);
 }
 
 template int gmres_apply_resident<double>(Solver *, Vec *, Vec *, int, bool, int *);

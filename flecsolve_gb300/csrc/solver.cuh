@@ -129,6 +129,8 @@ struct Solver {
 	ResSlots *res_slots = nullptr;
 	ulonglong2 *res_pk = nullptr;
 	void *res_vals = nullptr;
+	size_t res_vals_len = 0;
+	int res_polls = 0;  // reads after which they give up a wait (0: the default)
 	// captured graphs, keyed by the operator they were captured with and the
 	// vectors / body they run; at most kMaxGraphs are kept (least recently
 	// launched evicted first)
