@@ -216,7 +216,7 @@ _PROTOS = {
     "fs_krylov_settings_set": [_vp, C.POINTER(KrylovSettings)],
     "fs_krylov_apply": [_vp, _vp, _vp, C.POINTER(SolveInfo)],
     "fs_krylov_history": [_vp, _dp, C.POINTER(_i64)],
-    "fs_krylov_wait_limit": [_vp, C.c_int],
+    "fs_krylov_lose_cta": [_vp, C.c_int],
     "fs_krylov_mixed_stats": [_vp, C.POINTER(C.c_int), C.POINTER(C.c_int)],
     "fs_batch_cg_solve": [_vp, C.POINTER(KrylovSettings), _vp, C.c_int, C.POINTER(_i64), _vp, _vp,
                           C.c_int, C.c_int, C.POINTER(SolveInfo)],

@@ -681,10 +681,10 @@ class BoundSolver:
         check(lib().fs_krylov_history(self.h, out.ctypes.data_as(_lib._dp), C.byref(m)), self.ctx.h)
         return out[: m.value]
 
-    def wait_limit(self, reads: int) -> None:
-        """Looks at another CTA's message after which a solve in one
-        cooperative launch gives up with an error (0: the default)."""
-        check(lib().fs_krylov_wait_limit(self.h, int(reads)), self.ctx.h, "fs_krylov_wait_limit")
+    def lose_cta(self, cta: int) -> None:
+        """For tests of failure detection: CTA ``cta`` of a solve in one
+        cooperative launch leaves at once (-1: none does)."""
+        check(lib().fs_krylov_lose_cta(self.h, int(cta)), self.ctx.h, "fs_krylov_lose_cta")
 
     def mixed_stats(self):
         o, i = C.c_int(), C.c_int()

@@ -2444,13 +2444,13 @@ FS_API int fs_krylov_history(fs_solver h, double *hist, int64_t *n) {
 	return FS_OK;
 }
 
-FS_API int fs_krylov_wait_limit(fs_solver h, int reads) {
+FS_API int fs_krylov_lose_cta(fs_solver h, int cta) {
 	Solver *s = reinterpret_cast<Solver *>(h);
 	if (!ok_slv(s))
 		return FS_ERR_BAD_HANDLE;
-	if (reads < 0)
-		return set_err(s->ctx, FS_ERR_INVALID_ARG, "fs_krylov_wait_limit: negative limit");
-	s->res_polls = reads;
+	if (cta < -1 || cta >= (1 << 20))
+		return set_err(s->ctx, FS_ERR_INVALID_ARG, "fs_krylov_lose_cta: no such CTA");
+	s->res_lost = cta + 1;
 	return FS_OK;
 }
 

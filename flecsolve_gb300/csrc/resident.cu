@@ -34,7 +34,7 @@ struct ResCg {
 	int maxiter, hist_cap, zero_guess;
 	int rows;                 // rows per CTA
 	int smem;                 // dynamic shared memory, bytes
-	int polls;
+	int lost;
 };
 
 // PKT: the slice's p fits in shared memory and the other slices read it as
@@ -52,8 +52,10 @@ k_cg_resident(ResCg a) {
 		int turn;  // CTA that keeps the next entry of the history
 	};
 	__shared__ Scalars z;
+	if ((int)blockIdx.x == a.lost)
+		return;  // a test of the others' waits
 	ResTeam tm;
-	tm.init(a.slots, &sh, a.err, a.polls);
+	tm.init(a.slots, &sh, a.err);
 	const int tid = threadIdx.x, nt = blockDim.x;
 	const int lo = (int)min((int64_t)blockIdx.x * a.rows, (int64_t)a.A.n);
 	const int cnt = (int)min((int64_t)a.rows, (int64_t)a.A.n - lo);
@@ -344,7 +346,7 @@ int cg_apply_resident(Solver *s, Vec *b, Vec *x, fs_solve_info *info, int *taken
 	a.hist = s->hist;
 	a.slots = s->res_slots;
 	a.err = ctx->dev_err;
-	a.polls = res_polls(s);
+	a.lost = s->res_lost - 1;
 	a.rtol = (double)s->set.base.rtol;
 	a.maxiter = s->set.base.maxiter;
 	a.hist_cap = s->hist_cap;

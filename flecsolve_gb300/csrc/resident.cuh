@@ -26,11 +26,12 @@
 // A kernel whose packets did not flow into its next sum would need a fence.
 //
 // The launch is cooperative, so all CTAs are resident and every wait ends; as
-// a guard the waits are bounded all the same (kResPolls reads, or the solver's
-// own limit), after which the CTA records an error in the context's device
-// error word and leaves, as do the others when their own waits run out.  The
-// host then clears all messages (res_read_state): a CTA that began late may
-// have sent some of an epoch that the next launch would use.
+// a guard the waits are bounded all the same (kResPolls reads), after which the
+// CTA records an error in the context's device error word and leaves, as do the
+// others when their own waits run out.  (The bound is a constant: as a variable
+// it costs CG 4 % and the FP32 GMRES 10 %.)  The host then clears all messages
+// (res_read_state): CTA 0 may not have stored its last epoch, or a CTA that
+// began late may have sent some of an epoch that the next launch would use.
 #pragma once
 
 #include <algorithm>
@@ -44,7 +45,7 @@ namespace fsg {
 constexpr int kResMaxG = 160;      // CTAs of a resident grid at most
 constexpr int kResMaxVals = 4;     // values per grid_sum at most
 constexpr int kResThreads = 512;   // threads per CTA at most
-constexpr int kResPolls = 1 << 22;  // reads of a wait at most (some 300 ns each)
+constexpr int kResPolls = 1 << 22;  // reads of a wait at most (0.8 s in all)
 
 // ------------------------------------------------ sums in fixed point --
 //
@@ -327,7 +328,6 @@ struct ResShared {
 	ResFix part[kResMaxVals][kResThreads / 32];
 	double bc[8];  // scalars handed from warp 0 to the CTA
 	int stop;      // set by warp 0: leave the iteration loop
-	int polls;     // reads of a wait at most
 	int fail;      // a wait ran out
 };
 
@@ -369,8 +369,7 @@ struct ResTeam {
 	unsigned *err;
 	unsigned long long epoch;  // the same in every thread of the grid
 
-	// a CTA barrier follows before the first wait
-	__device__ void init(ResSlots *s, ResShared *shared, unsigned *e, int polls) {
+	__device__ void init(ResSlots *s, ResShared *shared, unsigned *e) {
 		slots = s;
 		sh = shared;
 		err = e;
@@ -378,7 +377,6 @@ struct ResTeam {
 		if (threadIdx.x == 0) {
 			sh->stop = 0;
 			sh->fail = 0;
-			sh->polls = polls;
 		}
 	}
 	__device__ void failed() {
@@ -392,7 +390,7 @@ struct ResTeam {
 		constexpr int Q = kResMaxG / 32;
 		const int lane = threadIdx.x & 31, G = (int)gridDim.x;
 		bool here = false;
-		for (int it = 0; !here && it < sh->polls; ++it) {
+		for (int it = 0; !here && it < kResPolls; ++it) {
 			// every slot of this lane in flight, then the tags
 			ulonglong2 m[Q];
 #pragma unroll
@@ -561,7 +559,7 @@ __device__ __forceinline__ bool widens(double) { return true; }
 // function: inlined, the loops of a row's neighbours cost the caller spills)
 static __device__ __noinline__ unsigned long long res_await(const ulonglong2 *p, unsigned long long tag,
                                                      ResShared *sh, unsigned *err) {
-	for (int it = 0; it < sh->polls && !*(volatile int *)&sh->fail; ++it) {
+	for (int it = 0; it < kResPolls && !*(volatile int *)&sh->fail; ++it) {
 		const ulonglong2 m = res_ld16(p);
 		if (m.y == tag)
 			return m.x;
@@ -849,7 +847,6 @@ inline bool res_grid(const Csr *A, ResGrid<V> &g, bool &gen) {
 // kernels, which need neither, run instead
 bool res_memory(Solver *s, bool packets);
 
-inline int res_polls(const Solver *s) { return s->res_polls > 0 ? s->res_polls : kResPolls; }
 // read_state after a resident kernel (resident.cu); clears all messages when a
 // wait ran out, so that the solver can be used again
 int res_read_state(Solver *s);

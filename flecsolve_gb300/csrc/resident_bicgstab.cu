@@ -29,7 +29,7 @@ struct ResBi {
 	unsigned *err;
 	double rtol;
 	int maxiter, hist_cap, zero_guess;
-	int rows, smem, polls;
+	int rows, smem, lost;
 };
 
 template<int K, bool GEN>
@@ -46,8 +46,10 @@ k_bi_resident(ResBi a) {
 	};
 	__shared__ Scalars z;
 	__shared__ ResRows<double, K, GEN> A;
+	if ((int)blockIdx.x == a.lost)
+		return;  // a test of the others' waits
 	ResTeam tm;
-	tm.init(a.slots, &sh, a.err, a.polls);
+	tm.init(a.slots, &sh, a.err);
 	const int tid = threadIdx.x, nt = blockDim.x;
 	const int lo = (int)min((int64_t)blockIdx.x * a.rows, (int64_t)a.A.n);
 	const int cnt = (int)min((int64_t)a.rows, (int64_t)a.A.n - lo);
@@ -440,7 +442,7 @@ int bicgstab_apply_resident(Solver *s, Vec *b, Vec *x, int *taken) {
 	a.hist = s->hist;
 	a.slots = s->res_slots;
 	a.err = ctx->dev_err;
-	a.polls = res_polls(s);
+	a.lost = s->res_lost - 1;
 	a.rtol = (double)s->set.base.rtol;
 	a.maxiter = s->set.base.maxiter;
 	a.hist_cap = s->hist_cap;

@@ -52,7 +52,7 @@ struct ResGm {
 	double *hist;
 	double rtol;
 	int maxiter, hist_cap, zero_guess, right, m, mixed;
-	int rows, smem, polls;
+	int rows, smem, lost;
 };
 
 // rows a thread takes at a time in the basis passes: 16 bytes of FP32 rows
@@ -229,8 +229,10 @@ k_gm_resident(ResGm<T> a) {
 	__shared__ RgSmall g;
 	__shared__ T *col[kGmDelayedCols];    // the slice's rows of each column
 	__shared__ T hs[kGmDelayedCols], ht[kGmDelayedCols];
+	if ((int)blockIdx.x == a.lost)
+		return;  // a test of the others' waits
 	ResTeam tm;
-	tm.init(a.slots, &sh, a.err, a.polls);
+	tm.init(a.slots, &sh, a.err);
 	const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5;
 	const int nwk = (nt >> 5) - 1, ntk = nwk * 32;  // workers; the last warp keeps the Hessenberg
 	const bool worker = wid < nwk;
@@ -485,7 +487,7 @@ k_gm_resident(ResGm<T> a) {
 					double q[2] = {0.0, 0.0};
 					bool here = false;
 					res_hold(clock64());
-					for (int it = 0; !here && it < sh.polls; ++it) {
+					for (int it = 0; !here && it < kResPolls; ++it) {
 						ulonglong2 m[2];
 #pragma unroll
 						for (int i = 0; i < 2; ++i)
@@ -771,7 +773,7 @@ int gmres_apply_resident(Solver *s, Vec *b, Vec *x, int m, bool mixed, int *take
 	a.vals = (RgSlots *)s->res_vals;
 	a.slots = s->res_slots;
 	a.err = ctx->dev_err;
-	a.polls = res_polls(s);
+	a.lost = s->res_lost - 1;
 	a.st = s->st;
 	a.hist = s->hist;
 	a.rtol = (double)s->set.base.rtol;

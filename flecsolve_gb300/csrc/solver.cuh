@@ -130,7 +130,7 @@ struct Solver {
 	ulonglong2 *res_pk = nullptr;
 	void *res_vals = nullptr;
 	size_t res_vals_len = 0;
-	int res_polls = 0;  // reads after which they give up a wait (0: the default)
+	int res_lost = 0;  // fs_krylov_lose_cta, counted from 1
 	// captured graphs, keyed by the operator they were captured with and the
 	// vectors / body they run; at most kMaxGraphs are kept (least recently
 	// launched evicted first)

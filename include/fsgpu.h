@@ -439,11 +439,11 @@ FS_API int fs_krylov_history(fs_solver s, double *hist, int64_t *n);
 /* number of refinement (outer) steps and total inner iterations of the last
  * FS_CG_MIXED apply */
 FS_API int fs_krylov_mixed_stats(fs_solver s, int *outer, int *inner_iters);
-/* A solve that runs as one cooperative launch waits for the other CTAs'
- * messages; after `reads` looks at one (0: the default, 2^22, a second or so)
- * it gives up, the apply returns FS_ERR_CUDA and x is undefined.  The solver
- * stays usable.  A small limit makes every such solve fail. */
-FS_API int fs_krylov_wait_limit(fs_solver s, int reads);
+/* For tests of failure detection: in the solves that run as one cooperative
+ * launch of several CTAs, CTA `cta` leaves at once (-1: none does).  The others
+ * wait for its messages until their limit (2^22 looks, 0.8 s), the
+ * apply then returns FS_ERR_CUDA, x is undefined, and the solver stays usable. */
+FS_API int fs_krylov_lose_cta(fs_solver s, int cta);
 
 /* ------------------------------------------------------------ adjoint --- */
 /* No counterpart in the reference (it has no adjoint).  For a loss L(x) of
