@@ -115,16 +115,11 @@ struct RgAcc<float> {
 };
 
 // the CTA's copy of the small state (the same in every CTA)
-//
-// A step's scalars have a slot for each parity: the Hessenberg warp reads those
-// of step k until it joins the barrier of step k + 1, while warp 0 may already
-// write those of step k + 1; step k + 2 writes after that barrier.
-struct RgStep {
-	double s[kGmDelayedCols], t[kGmDelayedCols];       // totals
-	double r, rinv, tau;
-};
 struct RgSmall {
-	RgStep step[2];
+	// of the step: the totals, r, 1 / r and tau.  The Hessenberg warp reads them
+	// beside the next step's passes; warp 0 writes the next ones after it is
+	// through (rg_read_done, rg_read_wait).
+	double s[kGmDelayedCols], t[kGmDelayedCols], r, rinv, tau;
 	double Hr[kGmDelayedCols * kGmDelayedCols];        // Hessenberg before the rotations
 	double H[kGmDelayedCols * kGmDelayedCols];         // and after
 	double cs[kGmDelayedCols], sn[kGmDelayedCols], dw[kGmDelayedCols + 1], dy[kGmDelayedCols];
@@ -140,22 +135,32 @@ __device__ __forceinline__ void rg_bar(int threads) {
 	asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
 }
 
+// The Hessenberg warp has read the step's scalars; warp 0, before it writes the
+// next ones.  us a step with this / with a slot for each parity of the step: FP64
+// 13.7 / 13.9 at 128^2, 13.7 / 14.1 at 64^2, FP32 13.5 / 14.0 at 32^3, 21.3 / 21.1
+// at 64^3.
+__device__ __forceinline__ void rg_read_done() {
+	__threadfence_block();
+	asm volatile("bar.arrive 2, 64;" ::: "memory");
+}
+__device__ __forceinline__ void rg_read_wait() { asm volatile("bar.sync 2, 64;" ::: "memory"); }
+
 // column c of the Hessenberg matrix is final up to the step's s and r:
 // rotations, estimate and stop tests (finish_step_warp of gmres.cu on the
 // CTA's copy; only CTA 0 writes the history)
-__device__ void rg_finish_column(RgSmall &g, const RgStep &st, int c, double *hist, int hist_cap,
-                                 int maxiter, int m, int mixed, int *flag) {
+__device__ void rg_finish_column(RgSmall &g, int c, double *hist, int hist_cap, int maxiter, int m,
+                                 int mixed, int *flag) {
 	constexpr int ld = kGmDelayedCols;
 	const int lane = threadIdx.x & 31;
 	double *col = g.H + ld * c;
 	if (lane < c + 1) {
-		const double h = g.Hr[lane + ld * c] + st.s[lane];
+		const double h = g.Hr[lane + ld * c] + g.s[lane];
 		g.Hr[lane + ld * c] = h;
 		col[lane] = h;
 	}
 	if (lane == 0) {
-		g.Hr[c + 1 + ld * c] = st.r;
-		col[c + 1] = st.r;
+		g.Hr[c + 1 + ld * c] = g.r;
+		col[c + 1] = g.r;
 	}
 	__syncwarp();
 	double x = col[0];
@@ -168,7 +173,7 @@ __device__ void rg_finish_column(RgSmall &g, const RgStep &st, int c, double *hi
 		x = __shfl_sync(0xffffffffu, v, 1);
 	}
 	if (lane == 0) {
-		const double gg = st.r;
+		const double gg = g.r;
 		col[c] = x;
 		// a column without a remainder takes the identity: its estimate
 		// is 0 and not what the cycle before left in dw[c + 1]
@@ -400,7 +405,6 @@ k_gm_resident(ResGm<T> a) {
 		for (int k = 0;; ++k) {
 			const bool last = k == a.m;  // u_m's sums alone finish the cycle
 			const int nv = last ? k + 1 : 2 * (k + 1);
-			RgStep &st = g.step[k & 1];
 			++tm.epoch;
 			if (worker) {
 				if (!last) {
@@ -509,18 +513,20 @@ k_gm_resident(ResGm<T> a) {
 						ss += __shfl_xor_sync(0xffffffffu, ss, o);
 						sw += __shfl_xor_sync(0xffffffffu, sw, o);
 					}
+					if (k > 0)
+						rg_read_wait();  // (no step precedes the first of a cycle)
 					if (lane <= k) {
-						st.s[lane] = q[0];
-						st.t[lane] = q[1];
+						g.s[lane] = q[0];
+						g.t[lane] = q[1];
 						hs[lane] = (T)q[0];
 						ht[lane] = (T)q[1];
 					}
 					const double r = k > 0 ? gm_norm(alpha - ss) : 1.0;
 					const double rinv = r != 0.0 ? 1.0 / r : 1.0;
 					if (lane == 0) {
-						st.r = r;
-						st.rinv = rinv;
-						st.tau = (gamma - sw) * rinv;
+						g.r = r;
+						g.rinv = rinv;
+						g.tau = (gamma - sw) * rinv;
 					}
 				}
 			}
@@ -536,17 +542,19 @@ k_gm_resident(ResGm<T> a) {
 			}
 			if (!worker) {
 				if (k > 0)
-					rg_finish_column(g, st, k - 1, a.hist, a.hist_cap, a.maxiter, a.m, a.mixed,
+					rg_finish_column(g, k - 1, a.hist, a.hist_cap, a.maxiter, a.m, a.mixed,
 					                 &g.flag[k & 1]);
 				if (!last && lane <= k) {
 					// tentative column k: ([t; tau] - H s) / r over rows 0..k
 					double d = 0.0;
 					for (int j = 0; j < k; ++j)
 						if (j + 1 >= lane)
-							d = fma(g.Hr[lane + kGmDelayedCols * j], st.s[j], d);
-					g.Hr[lane + kGmDelayedCols * k] = ((lane < k ? st.t[lane] : st.tau) - d) * st.rinv;
+							d = fma(g.Hr[lane + kGmDelayedCols * j], g.s[j], d);
+					g.Hr[lane + kGmDelayedCols * k] = ((lane < k ? g.t[lane] : g.tau) - d) * g.rinv;
 				}
 				__syncwarp();
+				if (!last)
+					rg_read_done();
 			}
 			if (last) {
 				__syncthreads();
@@ -557,7 +565,7 @@ k_gm_resident(ResGm<T> a) {
 			if (worker) {
 				// q_k = (u_k - Q s) / r, u_{k+1} = (w - Q t - tau q_k) / r
 				T *uk = col[k], *un = col[k + 1];
-				const T inv = (T)st.rinv, tau = (T)-st.tau;
+				const T inv = (T)g.rinv, tau = (T)-g.tau;
 				tag = tm.epoch;
 				for (int c = tid; c < nch; c += ntk) {
 					T q[W], n[W];
