@@ -1975,12 +1975,13 @@ static int bi_body32(Solver *s, void *a) {
 	      *t = s->w32[5], *xs = s->w32[6];
 	const float *dinv = PK == 1 ? s->dinv32() : nullptr;
 	const int G = red_grid(ctx, n);
+	const double around = 5.0 * sizeof(float) * (double)n;  // an iteration's vectors besides two
 	auto spmv = [&](const float *x, const auto &epi) -> int {
 		if constexpr (PK == 2)
 			return launch_spmv_grid<float, false, true>(ctx, s->A, GatherX<float>{x}, epi,
-			                                            (const float *)s->scaled);
+			                                            (const float *)s->scaled, around);
 		else
-			return launch_spmv<float, false, PK == 1>(ctx, s->A, s->A->val32, x, dinv, epi);
+			return launch_spmv<float, false, PK == 1>(ctx, s->A, s->A->val32, x, dinv, epi, around);
 	};
 	// plain launches: let in early, the next pass costs the running one more
 	// than its own start (96^3: 47.9 us an iteration with programmatic launches,

@@ -44,7 +44,7 @@ struct CsrGrid {
 constexpr int kGridThreads = 256;
 constexpr int kGridChunk = 4;
 
-template<class V, bool EXACT, bool GEN, class G, class Epi>
+template<class V, bool EXACT, bool GEN, bool ONCE, class G, class Epi>
 __global__ void __launch_bounds__(kGridThreads)
 spmv_grid_kernel(CsrGrid<V> A, G g_in, Epi epi) {
 	constexpr int NV = Epi::NV;
@@ -62,7 +62,13 @@ spmv_grid_kernel(CsrGrid<V> A, G g_in, Epi epi) {
 	const int nstep = (nseg + kGridThreads - 1) / kGridThreads;
 	const int segs_per_line = A.nx / W;
 	const int64_t nxy = (int64_t)A.nx * A.ny;
-	const unsigned long long once = once_policy();
+	const unsigned long long policy = ONCE ? once_policy() : 0;
+	auto load = [&](const V *p, V(&o)[W]) {
+		if constexpr (ONCE)
+			ld_vec16_once(p, o, policy);
+		else
+			ld_vec16(p, o);
+	};
 	const bool has_y = A.K >= 2, has_z = A.K >= 3;
 	const V *__restrict__ D = A.S;
 	const V *__restrict__ U1 = A.S + A.ld;
@@ -92,17 +98,11 @@ spmv_grid_kernel(CsrGrid<V> A, G g_in, Epi epi) {
 		V d[W], u1[W], u2[W], u3[W], u2m[W], u3m[W], l1[W];
 		V x[W], xmy[W], xpy[W], xmz[W], xpz[W];
 		V u1m = V(0), xm1 = V(0), xp1 = V(0);
-		if constexpr (GEN) {
-			ld_vec16_once(D + r0, d, once);
-			ld_vec16_once(U1 + r0, u1, once);
-		}
-		else {
-			ld_vec16(D + r0, d);
-			ld_vec16(U1 + r0, u1);
-		}
+		load(D + r0, d);
+		load(U1 + r0, u1);
 		g.at_vec(r0, x);
 		if constexpr (GEN)
-			ld_vec16_once(L1 + r0, l1, once);
+			load(L1 + r0, l1);
 		if (lo_x) {
 			if constexpr (!GEN)
 				u1m = __ldg(U1 + r0 - 1);
@@ -111,30 +111,18 @@ spmv_grid_kernel(CsrGrid<V> A, G g_in, Epi epi) {
 		if (hi_x)
 			xp1 = g.at(r0 + W);
 		if (has_y) {
-			if constexpr (GEN)
-				ld_vec16_once(U2 + r0, u2, once);
-			else
-				ld_vec16(U2 + r0, u2);
+			load(U2 + r0, u2);
 			if (lo_y) {
-				if constexpr (GEN)
-					ld_vec16_once(L2 + r0, u2m, once);
-				else
-					ld_vec16(U2 + r0 - A.nx, u2m);
+				load(GEN ? L2 + r0 : U2 + (r0 - A.nx), u2m);
 				g.at_vec(r0 - A.nx, xmy);
 			}
 			if (hi_y)
 				g.at_vec(r0 + A.nx, xpy);
 		}
 		if (has_z) {
-			if constexpr (GEN)
-				ld_vec16_once(U3 + r0, u3, once);
-			else
-				ld_vec16(U3 + r0, u3);
+			load(U3 + r0, u3);
 			if (lo_z) {
-				if constexpr (GEN)
-					ld_vec16_once(L3 + r0, u3m, once);
-				else
-					ld_vec16(U3 + (r0 - nxy), u3m);
+				load(GEN ? L3 + r0 : U3 + (r0 - nxy), u3m);
 				g.at_vec((int)(r0 - nxy), xmz);
 			}
 			if (hi_z)
@@ -206,23 +194,35 @@ inline const double *gen_vals<double>(const Csr *A) { return A->gen64; }
 template<>
 inline const float *gen_vals<float>(const Csr *A) { return A->gen32; }
 
-// `vals`: other values in A's storage
+// Bytes that a loop's pass over values and vectors cycles through from which
+// the general storage's values leave the L2 (129 MB) first.  us without / with,
+// SpMV after SpMV: FP32 96^3 (32 MB) 4.7 / 5.0, 128^3 (75) 7.8 / 10.5, 136^3 (91)
+// 12.7 / 14.6, 144^3 (108) 17.2 / 16.5, 192^3 (255) 39.7 / 33.5; FP64 96^3 (64) 13.0
+// / 13.8, 104^3 (81) 22.6 / 23.3, 112^3 (101) 26.9 / 26.7, 160^3 (295) 61.8 / 60.6.
+// An iteration of mixed BiCGSTAB: 112^3 (79) 51.3 / 53.2, 128^3 (117) 81.6 / 77.1; of
+// FP64 BiCGSTAB 120^3 (124) 188 / 182.
+constexpr double kOnceBytes = 100e6;
+
+// `vals`: other values in A's storage; `around`: bytes of the vectors besides x
+// and y that the caller's loop cycles through
 template<class V, bool EXACT, bool GEN, class G, class Epi>
 static inline int launch_spmv_grid(Ctx *ctx, const Csr *A, const G &g, const Epi &epi,
-                                   const V *vals = nullptr) {
-	static int per_sm = 0;  // resident CTAs per SM of this instantiation
+                                   const V *vals = nullptr, double around = 0.0) {
+	static int per_sm[2] = {0, 0};  // resident CTAs per SM of these instantiations
 	constexpr int W = 16 / (int)sizeof(V);
-	auto kern = spmv_grid_kernel<V, EXACT, GEN, G, Epi>;
-	if (per_sm == 0) {
+	const bool once = GEN && (2.0 * A->nsym + 3.0) * (double)A->nrows * sizeof(V) + around >= kOnceBytes;
+	auto kern = once ? spmv_grid_kernel<V, EXACT, GEN, GEN, G, Epi>
+	                 : spmv_grid_kernel<V, EXACT, GEN, false, G, Epi>;
+	if (per_sm[once] == 0) {
 		int nb = 0;
 		if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, kGridThreads, 0) != cudaSuccess ||
 		    nb < 1)
 			nb = 1;
-		per_sm = nb;
+		per_sm[once] = nb;
 	}
 	const int nseg = (int)(A->nrows / W);
 	const int nstep = (nseg + kGridThreads - 1) / kGridThreads;
-	const int resident = ctx->sms * std::min(per_sm, 8);
+	const int resident = ctx->sms * std::min(per_sm[once], 8);
 	const int chunk = nstep >= kGridChunk * resident ? kGridChunk : 1;
 	const int nchunk = (nstep + chunk - 1) / chunk;
 	const int grid = std::max(1, std::min(nchunk, resident));

@@ -192,8 +192,7 @@ __device__ __forceinline__ void ld_vec16(const double *p, double (&o)[2]) {
 
 // the same for values that a kernel reads once: not kept in the L1, first to
 // leave the L2, so that the vectors between two passes stay there instead
-// (mixed BiCGSTAB's iteration at 192^3 172.7 -> 162.0 us, at 128^3 81.5 -> 76.8,
-// at 96^3, where all of it stays, 42.3 -> 42.5)
+// (kOnceBytes in spmv_grid.cuh says when)
 __device__ __forceinline__ unsigned long long once_policy() {
 	unsigned long long p;
 	asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
@@ -480,7 +479,7 @@ namespace fsg {
 // kernel when the matrix carries patterns, else column ids.
 template<class V, bool EXACT, bool SCALE, class Epi>
 static inline int launch_spmv(Ctx *ctx, const Csr *A, const V *vals, const V *x,
-                              const V *dscale, const Epi &epi) {
+                              const V *dscale, const Epi &epi, double around = 0.0) {
 	constexpr bool F32 = std::is_same_v<V, float>;
 	if (A->fvm) {  // matrix-free finite-volume operator
 		if constexpr (SCALE)
@@ -498,9 +497,9 @@ static inline int launch_spmv(Ctx *ctx, const Csr *A, const V *vals, const V *x,
 	}
 	if (coding == kCodingGridGen && own_vals && grid_aligned<V>(A, x, dscale)) {
 		if constexpr (SCALE)
-			return launch_spmv_grid<V, EXACT, true>(ctx, A, GatherScale<V>{x, dscale}, epi);
+			return launch_spmv_grid<V, EXACT, true>(ctx, A, GatherScale<V>{x, dscale}, epi, nullptr, around);
 		else
-			return launch_spmv_grid<V, EXACT, true>(ctx, A, GatherX<V>{x}, epi);
+			return launch_spmv_grid<V, EXACT, true>(ctx, A, GatherX<V>{x}, epi, nullptr, around);
 	}
 	if ((coding == kCodingSym || coding == kCodingGrid) && own_vals) {
 		if constexpr (SCALE)

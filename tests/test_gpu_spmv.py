@@ -386,3 +386,23 @@ def test_solvers_over_vector_spmv(ctx, lanes, method):
     assert abs(info.iters - ref.iters) <= 2
     x = vx.numpy()
     assert np.linalg.norm(b - A.to_scipy() @ x) <= 1.01e-10 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n", [108, 112, 140, 144])
+def test_general_grid_spmv_either_side_of_the_l2(ctx, n):
+    """Convection-diffusion below and above the bytes from which the values
+    leave the L2 first (FP64 from 112^3, FP32 from 141^3 on): the bits of the
+    row patterns, in both types and exact modes."""
+    A = P.convdiff3d(n, seed=4)
+    got = {}
+    x = P.uniform(5, A.nrows)
+    for coding in ("grid", "patterns"):
+        dA = fs.CSR(ctx, A)
+        dA.index_coding(coding)
+        for dtype, exact in (("f64", False), ("f64", True), ("f32", False)):
+            vx = fs.Vector(ctx, x.astype(np.float32 if dtype == "f32" else np.float64), dtype=dtype)
+            vy = fs.Vector(ctx, A.nrows, dtype=dtype)
+            dA.apply(vx, vy, exact=exact)
+            got[coding, dtype, exact] = vy.numpy()
+    for dtype, exact in (("f64", False), ("f64", True), ("f32", False)):
+        assert np.array_equal(got["grid", dtype, exact], got["patterns", dtype, exact])
