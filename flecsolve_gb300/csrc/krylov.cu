@@ -1570,10 +1570,13 @@ struct RcArgs {
 	double delta;
 };
 
-// Rows from which the passes of mixed CG alternate direction: us an iteration
-// forwards / alternating 27.6 / 27.9 at 64^3, 35.7 / 36.0 at 96^3, 75.3 / 76.0 at
-// 160^3, 127.6 / 127.2 at 200^3, 216.5 / 214.1 at 256^3.  While an iteration's 64
-// bytes a row fit twice in the L2, both orders find what the last pass left.
+// Rows from which the passes of mixed CG alternate direction, where the SpMV can
+// (the grid kernel): us an iteration forwards / alternating 27.6 / 27.9 at 64^3,
+// 35.7 / 36.0 at 96^3, 75.3 / 76.0 at 160^3, 123.7 / 123.7 at 200^3, 157.5 / 155.8 at
+// 224^3, 213.9 / 211.7 at 256^3, 347.2 / 345.4 at 300^3 (runs of one side differ by
+// 0.1).  While an iteration's 64 bytes a row fit twice in the L2, both orders find
+// what the last pass left.  The other two passes alone, against an SpMV that walks
+// forwards (255^3), lose: 243.4 / 244.5.
 constexpr int64_t kTurnRows = 6000000;
 
 template<int PK>
@@ -1590,7 +1593,8 @@ static int rc_body(Solver *s, void *a) {
 	// direction pass on the residual pass's last r and D^-1, the next SpMV on
 	// the direction pass's last p (a body of an odd count starts like an even
 	// one; only the first pass of the next body then misses).
-	const bool turn = n >= kTurnRows;
+	const int coding = active_coding(s->A, true);
+	const bool turn = n >= kTurnRows && !s->A->fvm && (coding == kCodingGrid || coding == kCodingGridGen);
 	for (int k = 0; k < g->k; ++k) {
 		const bool back = turn && (k & 1), rback = turn && !back;
 		FS_TRY(launch_spmv<float, false, false>(
