@@ -710,10 +710,11 @@ def batch_cg(A: CSR, offsets, b: Vector, x: Vector, maxiter: int, rtol: float,
              use_zero_guess: bool = True, delta: float = 0.0, cluster: int = 0,
              threads: int = 0, fp64_head: float = None, cluster_systems: int = None):
     """Solve the independent systems on the diagonal blocks of ``A`` (system
-    s = rows offsets[s]:offsets[s+1]) in one persistent launch, one thread-
-    block cluster per system; returns one :class:`SolveInfo` per system.
-    ``cluster``/``threads`` = 0 lets the autotuner choose; ``fp64_head``: FP64
-    iterations until each system's residual is below that fraction of its
+    s = rows offsets[s]:offsets[s+1]) in one call, one thread-block cluster
+    per system; returns one :class:`SolveInfo` per system.
+    ``cluster``/``threads`` = 0: symmetric 5-point systems on square grids run
+    on chip (:func:`batch_on_chip`), others as the autotuner chooses;
+    ``fp64_head``: FP64 iterations until each system's residual is below that fraction of its
     ||b|| (None: the library default, 3e-3; 0: FP32 from the start).
     ``cluster_systems`` (with explicit sizes): that many of the largest
     systems own a cluster, every other system one CTA."""
@@ -761,12 +762,23 @@ def batch_tuning(A: CSR, offsets):
 
 def batch_schedule(A: CSR, offsets):
     """(cluster size, threads per CTA, systems that own a cluster) the
-    autotuner chose for this partition."""
+    autotuner chose for this partition; after a solve on chip the explicit
+    schedule closest to it."""
     off = np.ascontiguousarray(offsets, dtype=np.int64)
     c, t, nb = C.c_int(), C.c_int(), C.c_int()
     check(lib().fs_batch_schedule(A.ctx.h, A.h, off.size - 1, off.ctypes.data_as(C.POINTER(C.c_int64)),
                                   C.byref(c), C.byref(t), C.byref(nb)), A.ctx.h, "fs_batch_schedule")
     return c.value, t.value, nb.value
+
+
+def batch_on_chip(A: CSR, offsets) -> int:
+    """Launches of the last :func:`batch_cg` on this partition if it kept every
+    system on chip, else 0."""
+    off = np.ascontiguousarray(offsets, dtype=np.int64)
+    k = C.c_int()
+    check(lib().fs_batch_on_chip(A.ctx.h, A.h, off.size - 1, off.ctypes.data_as(C.POINTER(C.c_int64)),
+                                 C.byref(k)), A.ctx.h, "fs_batch_on_chip")
+    return k.value
 
 
 def batch_format(A: CSR, offsets) -> str:

@@ -571,6 +571,7 @@ struct BatchPlan {
 	int tuned_cluster = 0, tuned_threads = 0;
 	int tuned_nbig = -1;  // systems that own a whole cluster (-1: all)
 	bool ruled = false;   // the three stand for `classes`, not for a tuning
+	int on_chip = 0;      // launches of the last call if it ran on chip
 	// grid-stencil storage (every system a 5-point s x s grid with symmetric
 	// values): per-system sides, diagonal and upper diagonals; `grid` is 1
 	// when it holds for the values of generation `grid_gen`, 0 when not, -1
@@ -894,6 +895,7 @@ int batch_solve(fs_ctx h, const fs_krylov_settings *s, fs_csr Ah, int nsys, cons
 	}
 
 	int cl = cluster_size, th = threads;
+	p.on_chip = 0;
 	if (!cl && !th && cluster_systems < 0 && p.grid == 1) {
 		if (!p.classed) {
 			std::vector<int> order(nsys);
@@ -912,6 +914,7 @@ int batch_solve(fs_ctx h, const fs_krylov_settings *s, fs_csr Ah, int nsys, cons
 				if (c.team > 1)
 					p.tuned_nbig = c.first + c.count;
 			FS_TRY(launch_classes(ctx, a, p));
+			p.on_chip = (int)p.classes.size();
 			FS_CUDA_TRY(ctx, cudaMemcpyAsync(infos, p.d_info, sizeof(fs_solve_info) * nsys,
 			                                 cudaMemcpyDeviceToHost, ctx->stream));
 			FS_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1081,6 +1084,20 @@ extern "C" FS_API int fs_batch_schedule(fs_ctx h, fs_csr Ah, int nsys, const int
 	std::vector<int64_t> off(sys_offsets, sys_offsets + nsys + 1);
 	const int nbig = g_plans.find(std::make_pair((const Csr *)A, off))->second.tuned_nbig;
 	*cluster_systems = nbig < 0 ? nsys : nbig;
+	return FS_OK;
+}
+
+extern "C" FS_API int fs_batch_on_chip(fs_ctx h, fs_csr Ah, int nsys, const int64_t *sys_offsets,
+                                       int *launches) {
+	Ctx *ctx = reinterpret_cast<Ctx *>(h);
+	Csr *A = reinterpret_cast<Csr *>(Ah);
+	if (!ok_ctx(ctx) || !ok_csr(A) || !sys_offsets || !launches || nsys < 1)
+		return FS_ERR_BAD_HANDLE;
+	std::vector<int64_t> off(sys_offsets, sys_offsets + nsys + 1);
+	auto it = g_plans.find(std::make_pair((const Csr *)A, off));
+	if (it == g_plans.end())
+		return set_err(ctx, FS_ERR_INVALID_ARG, "no batched solve has run on this partition");
+	*launches = it->second.on_chip;
 	return FS_OK;
 }
 

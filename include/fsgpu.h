@@ -464,18 +464,25 @@ FS_API int fs_fv_face_grad(fs_ctx ctx, int dim, int64_t n, fs_vec lambda, fs_vec
                            int accumulate, fs_vec grad_faces);
 
 /* --------------------------------------------------- batched solves --- */
-/* Many independent systems in one persistent launch (no counterpart in the
+/* Many independent systems in one call (no counterpart in the
  * reference, whose solvers take one system per call: this batches calls of
  * cg.hh:43-139).  A is block diagonal: system s owns rows and columns
  * [sys_offsets[s], sys_offsets[s+1]).  One thread-block cluster per system
  * runs Jacobi-PCG with FP32 values/vectors and FP64 residual replacement
  * (settings->inner_rtol = replacement factor), stopping per system on the
- * FP64 residual (rtol * ||b_s||).  cluster_size (1, 2, 4, 8) and threads per
- * CTA may be 0: an autotuner times the candidates on the first call for this
- * partition and keeps the fastest (fs_batch_tuning reports it).  With both 0
- * it also tries schedules where only the largest systems own a whole cluster
- * and every other system one CTA (fs_batch_schedule reports how many own a
- * cluster).  infos[s] receives system s's solve_info. */
+ * FP64 residual (rtol * ||b_s||).  infos[s] receives system s's solve_info.
+ *
+ * With cluster_size and threads both 0, a batch of symmetric 5-point systems
+ * on square grids (FS_BATCH_GRID below) of up to some 180,000 rows each is
+ * solved on chip, by rule and untimed: 1 to 16 CTAs a system, one launch for
+ * each cluster size (fs_batch_on_chip says so).  Every other call is one
+ * persistent launch of a general kernel.  Its cluster_size (1, 2, 4, 8) and
+ * threads per CTA may be 0: an autotuner times the candidates on the first call
+ * for this partition and keeps the fastest (fs_batch_tuning reports it); with
+ * both 0 it also tries schedules where only the largest systems own a whole
+ * cluster and every other system one CTA (fs_batch_schedule reports how many
+ * own a cluster).  After an on-chip solve those two report the explicit
+ * schedule closest to it, which did not run. */
 FS_API int fs_batch_cg_solve(fs_ctx ctx, const fs_krylov_settings *s, fs_csr A, int nsys,
                              const int64_t *sys_offsets, fs_vec b, fs_vec x, int cluster_size,
                              int threads, fs_solve_info *infos);
@@ -483,12 +490,15 @@ FS_API int fs_batch_tuning(fs_ctx ctx, fs_csr A, int nsys, const int64_t *sys_of
                            int *cluster_size, int *threads);
 FS_API int fs_batch_schedule(fs_ctx ctx, fs_csr A, int nsys, const int64_t *sys_offsets,
                              int *cluster_size, int *threads, int *cluster_systems);
+/* launches of the last call on this partition if it ran on chip, else 0 */
+FS_API int fs_batch_on_chip(fs_ctx ctx, fs_csr A, int nsys, const int64_t *sys_offsets, int *launches);
 /* The storage the batched kernel's row sums read for this partition, checked
  * on the first solve after the values change: FS_BATCH_GRID when every
  * system is a 5-point operator on a square s x s grid (rows hold exactly
  * their in-grid neighbours, columns sorted) whose lower entries equal their
  * partners bit for bit -- the diagonal and two upper diagonals are read,
- * no column ids, with the CSR row loop's bits -- else FS_BATCH_CSR. */
+ * no column ids; the general kernel has the CSR row loop's bits on it -- else
+ * FS_BATCH_CSR. */
 #define FS_BATCH_CSR 0
 #define FS_BATCH_GRID 1
 FS_API int fs_batch_format(fs_ctx ctx, fs_csr A, int nsys, const int64_t *sys_offsets, int *format);

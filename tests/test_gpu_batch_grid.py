@@ -88,3 +88,23 @@ def test_grid_batch_with_clusters_that_wait_for_room(ctx):
     for lo, hi in zip(off[:-1], off[1:]):
         assert np.linalg.norm(r[lo:hi]) <= 1e-5 * (1 + 1e-3) * np.linalg.norm(b[lo:hi])
     assert np.array_equal(xs[0], xs[1]) and np.array_equal(xs[0], xs[2])
+
+
+def test_batch_on_chip_says_which_kernel_ran(ctx):
+    """Squares with sizes left to the library: on chip, one launch for each
+    cluster size; explicit sizes and systems that are no squares: the general
+    kernel."""
+    A, off, b = _batch((20, 33, 131))
+    dA, vb, vx = fs.CSR(ctx, A), fs.Vector(ctx, b), fs.Vector(ctx, A.nrows)
+    run = lambda **kw: fs.batch_cg(dA, off, vb, vx, maxiter=50, rtol=1e-3, **kw)
+    for kw, ran in ((dict(), True), (dict(cluster=2, threads=256), False), (dict(), True), (dict(cluster=1), False),
+                    (dict(threads=512), False), (dict(cluster=2, threads=256, cluster_systems=1), False)):
+        run(**kw)
+        assert (fs.batch_on_chip(dA, off) > 0) == ran
+        if ran:
+            assert fs.batch_on_chip(dA, off) <= 3
+            assert fs.batch_schedule(dA, off)[0] in (1, 2, 4, 8)
+    M, moff = P.block_diagonal([P.diffusion(3, 9, seed=1), P.diffusion(2, 30, seed=2)])
+    dM = fs.CSR(ctx, M)
+    fs.batch_cg(dM, moff, fs.Vector(ctx, P.uniform(3, M.nrows)), fs.Vector(ctx, M.nrows), maxiter=50, rtol=1e-3)
+    assert fs.batch_on_chip(dM, moff) == 0
