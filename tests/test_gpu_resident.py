@@ -415,3 +415,30 @@ def test_waits_that_run_out_end_the_solve_with_an_error(ctx, method, kw, shape, 
         assert (info.status, info.iters) == (ref.status, ref.iters)
         assert np.array_equal(got.numpy(), want.numpy())
         assert np.array_equal(slv.history(), fresh.history())
+
+
+@pytest.mark.parametrize("shape", [(75, 77, 77), (75, 71, 73), (33, 35, 37)])
+@pytest.mark.parametrize("method,u", [("gmres", 2.0 ** -53), ("mixed_gmres", 2.0 ** -24)])
+def test_resident_gmres_estimate_on_odd_rows(ctx, method, u, shape):
+    """As test_resident_gmres_estimate_is_the_true_residual, on row counts that
+    are no multiple of 4 (the last group of four FP32 rows is short), most of
+    whose columns are in global memory, and into the second cycle."""
+    A = _grid(*shape, 3, seed=sum(shape))
+    b = P.uniform(3, A.nrows)
+    M = A.to_scipy()
+    D = M.diagonal()
+    dA, vb = fs.CSR(ctx, A), fs.Vector(ctx, b)
+    assert dA.index_coding("grid") is not None and A.nrows % 4
+    ns = getattr(fs, method)
+    for k in (1, 2, 13, 14, 15, 16, 29, 30, 37):
+        s = ns.settings(use_zero_guess=True, maxiter=k, rtol=1e-30, max_krylov_dim=30, restart=True, ortho="dcgs2")
+        vx = fs.Vector(ctx, A.nrows)
+        before = ctx.launches
+        slv = ns.solver(s, ns.make_work(vb))(fs.op.ref(dA), fs.op.jacobi)
+        slv(vb, vx)
+        assert ctx.launches - before < 8  # one launch, and the storage's
+        h, x = slv.history(), vx.numpy()
+        assert h.size == k
+        true = np.linalg.norm(b - M @ x)
+        bound = 16 * (min(k, 30) + 5) * u * (np.sqrt(min(k, 30)) * np.linalg.norm(D * x) + h[-1])
+        assert abs(h[-1] - true) <= bound, (k, h[-1], true, bound)
