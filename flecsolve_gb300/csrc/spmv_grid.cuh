@@ -113,7 +113,10 @@ spmv_grid_kernel(CsrGrid<V> A, G g_in, Epi epi) {
 		if (has_y) {
 			load(U2 + r0, u2);
 			if (lo_y) {
-				load(GEN ? L2 + r0 : U2 + (r0 - A.nx), u2m);
+				if constexpr (GEN)
+					load(L2 + r0, u2m);
+				else
+					load(U2 + r0 - A.nx, u2m);
 				g.at_vec(r0 - A.nx, xmy);
 			}
 			if (hi_y)
@@ -122,7 +125,10 @@ spmv_grid_kernel(CsrGrid<V> A, G g_in, Epi epi) {
 		if (has_z) {
 			load(U3 + r0, u3);
 			if (lo_z) {
-				load(GEN ? L3 + r0 : U3 + (r0 - nxy), u3m);
+				if constexpr (GEN)
+					load(L3 + r0, u3m);
+				else
+					load(U3 + (r0 - nxy), u3m);
 				g.at_vec((int)(r0 - nxy), xmz);
 			}
 			if (hi_z)
