@@ -1572,9 +1572,9 @@ struct RcArgs {
 
 // Rows from which the passes of mixed CG alternate direction, where the SpMV can
 // (the grid kernel): us an iteration forwards / alternating 27.6 / 27.9 at 64^3,
-// 35.7 / 36.0 at 96^3, 75.3 / 76.0 at 160^3, 123.7 / 123.7 at 200^3, 157.5 / 155.8 at
-// 224^3, 213.9 / 211.7 at 256^3, 347.2 / 345.4 at 300^3 (runs of one side differ by
-// 0.1).  While an iteration's 64 bytes a row fit twice in the L2, both orders find
+// 35.7 / 36.0 at 96^3, 75.3 / 76.0 at 160^3, 120.9 / 120.6 at 200^3, 155.0 / 152.8 at
+// 224^3, 209.2 / 206.8 at 256^3, 341.1 / 339.6 at 300^3 (runs of one side differ by
+// 0.05).  While an iteration's 64 bytes a row fit twice in the L2, both orders find
 // what the last pass left.  The other two passes alone, against an SpMV that walks
 // forwards (255^3), lose: 243.4 / 244.5.
 constexpr int64_t kTurnRows = 6000000;
