@@ -346,7 +346,7 @@ int cg_apply_resident(Solver *s, Vec *b, Vec *x, fs_solve_info *info, int *taken
 	a.hist = s->hist;
 	a.slots = s->res_slots;
 	a.err = ctx->dev_err;
-	a.lost = s->res_lost - 1;
+	a.lost = sh.grid > 1 ? s->res_lost - 1 : -1;
 	a.rtol = (double)s->set.base.rtol;
 	a.maxiter = s->set.base.maxiter;
 	a.hist_cap = s->hist_cap;

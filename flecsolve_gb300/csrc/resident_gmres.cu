@@ -718,9 +718,9 @@ k_gm_resident(ResGm<T> a) {
 }
 
 // Rows up to which GMRES runs resident, by the basis type.  us a step, kernels
-// -> resident.  FP64 (modified Gram-Schmidt in kernels): 128^2 120 -> 13.0,
+// -> resident.  FP64 (modified Gram-Schmidt in kernels): 128^2 120 -> 13.7,
 // 512^2 124 -> 45.7, 64^3 140 -> 46.6, 100^3 237 -> 162.  FP32 (the staged
-// passes): 32^3 28.3 -> 13.6, 64^3 32.1 -> 21.6, 96^3 52.9 -> 64.6: past 0.45 M
+// passes): 32^3 28.3 -> 13.5, 64^3 32.1 -> 21.3, 96^3 52.9 -> 64.6: past 0.45 M
 // rows the columns no longer fit and the tensor copies of the staged passes
 // stream them better than this kernel's loads.
 template<class T>
@@ -781,7 +781,7 @@ int gmres_apply_resident(Solver *s, Vec *b, Vec *x, int m, bool mixed, int *take
 	a.vals = (RgSlots *)s->res_vals;
 	a.slots = s->res_slots;
 	a.err = ctx->dev_err;
-	a.lost = s->res_lost - 1;
+	a.lost = sh.grid > 1 ? s->res_lost - 1 : -1;
 	a.st = s->st;
 	a.hist = s->hist;
 	a.rtol = (double)s->set.base.rtol;
