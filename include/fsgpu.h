@@ -176,7 +176,8 @@ FS_API int fs_csr_values_device_ptr(fs_csr A, double **dval);
  *  4 general grid stencil (active only, through a request of format 3): a
  *    grid stencil as in format 3 whose values are not symmetric, read from
  *    the diagonal, the upper diagonals and the lower diagonals a(r, r - d)
- *    stored at row r.
+ *    stored at row r.  The SpMV lets the values leave the L2 first where a pass
+ *    over values and vectors exceeds 100 MB.
  *  Formats 1-4 give the bits of format 0.
  * enable: 0 .. 3 requests a format (a matrix falls back to the best format it
  * supports), -1 leaves it unchanged; *active (may be NULL) = the format the
@@ -366,7 +367,8 @@ enum fs_gmres_side { FS_LEFT = 0, FS_RIGHT = 1 };
  * where DCGS2 cannot run) for the FP32 basis of FS_GMRES_MIXED: 2 passes and
  * 1 reduction per step instead of the k + 2 of MGS.  On a grid-stencil operator
  * of up to 1,000,000 rows (FS_GMRES_MIXED: 450,000) AUTO and DCGS2 run the whole
- * solve as one cooperative launch with DCGS2 (m <= 30, no diagnostic callback).
+ * solve as one cooperative launch with DCGS2 (m <= 30, no diagnostic callback;
+ * index format 3, the default; asymmetric values need nx a multiple of 4).
  * DCGS2: CGS2 with each vector's reorthogonalisation delayed to the next
  * step, where it shares that step's pass of dot products (two passes over
  * the basis a step instead of three); the convergence test of a step runs
